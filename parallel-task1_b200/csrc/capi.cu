@@ -774,6 +774,11 @@ int trav_bellman_ford_el_f32(const int32_t *src, const int32_t *dst, const float
     trav_graph *h = nullptr;
     TRY(new_handle(&h));
     std::unique_ptr<trav_graph, void (*)(trav_graph *)> guard(h, destroy);
+    // sweeps over the edge list; a graph that needs more of them than the CSR
+    // kernels would cost goes on from the distances reached so far
+    bool done = false;
+    TRY(el_bellman_ford_sweeps(src, dst, w, vertices, edges, d, h->st, &done));
+    if (done) return TRAV_OK;
     TRY(build_graph_device(vertices, edges, src, dst, w, h->st, &h->g));
     TRY(workspace_ensure(&h->ws, h->g, 1, h->st));
     gather_bits_kernel<<<(vertices + 255) / 256 < 4096 ? (vertices + 255) / 256 : 4096, 256, 0, h->st>>>(
@@ -801,6 +806,10 @@ int trav_bfs_el(const int32_t *src, const int32_t *dst, int32_t vertices, int64_
     trav_graph *h = nullptr;
     TRY(new_handle(&h));
     std::unique_ptr<trav_graph, void (*)(trav_graph *)> guard(h, destroy);
+    // sweeps over the edge list; a graph with paths too long for them is built
+    bool done = false;
+    TRY(el_reach_sweeps(src, dst, vertices, edges, source, nullptr, 0, visited, h->st, &done));
+    if (done) return TRAV_OK;
     TRY(build_graph_device(vertices, edges, src, dst, nullptr, h->st, &h->g));
     TRY(workspace_ensure(&h->ws, h->g, 1, h->st));
     trav_bfs_opts o{TRAV_SCHEDULE_PLAIN, 15.0f, 18.0f, -1};
@@ -841,6 +850,9 @@ int trav_reach_el_masked(const int32_t *src, const int32_t *dst, int32_t vertice
     trav_graph *h = nullptr;
     TRY(new_handle(&h));
     std::unique_ptr<trav_graph, void (*)(trav_graph *)> guard(h, destroy);
+    bool done = false;
+    TRY(el_reach_sweeps(src, dst, vertices, edges, p, trees, want, visited, h->st, &done));
+    if (done) return TRAV_OK;
     TRY(build_graph_device(vertices, edges, src, dst, nullptr, h->st, &h->g));
     TRY(workspace_ensure(&h->ws, h->g, 1, h->st));
     DevTmp<int32_t> color;

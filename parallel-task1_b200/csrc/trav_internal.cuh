@@ -279,6 +279,14 @@ int rmat_device(int scale, int avg, int a, int b, int c, int d, uint32_t seed, i
 int validate_edges(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_dst, const float *d_w,
                    cudaStream_t st);
 
+// el_sweep.cu: one query on a device edge list, answered by sweeps over the
+// edges.  Waits for the result; *done = false: it would take too many sweeps
+// (the outputs are untouched, except that d may hold lower distances already).
+int el_reach_sweeps(const int32_t *src, const int32_t *dst, int32_t V, int64_t E, int32_t source, const int32_t *trees,
+                    int32_t want, uint8_t *visited, cudaStream_t st, bool *done);
+int el_bellman_ford_sweeps(const int32_t *src, const int32_t *dst, const float *w, int32_t V, int64_t E, float *d,
+                           cudaStream_t st, bool *done);
+
 // el_optimize.cu
 int el_optimize_device(int32_t *src, int32_t *dst, float *w, int64_t E, int32_t segment, int64_t *E_out,
                        cudaStream_t st);
