@@ -101,9 +101,9 @@ TeamLayout team_layout(const trav_batch *b)
 int release_teams(trav_batch *b)
 {
     TRY_CUDA(cudaStreamSynchronize(b->st));
-    cudaFree(b->team_mem);
-    cudaFree(b->d_teams);
-    cudaFree(b->ctl);
+    dev_free(b->team_mem);
+    dev_free(b->d_teams);
+    dev_free(b->ctl);
     b->team_mem = nullptr;
     b->d_teams = nullptr;
     b->ctl = nullptr;
@@ -333,7 +333,7 @@ int upload_queries(trav_batch *b, const trav_query *qs, int32_t n, int smooth_ta
     TRY(build_queries(b, qs, n, &d, smooth_tail));
     if (n > b->q_cap) {
         TRY_CUDA(cudaStreamSynchronize(b->st));
-        cudaFree(b->d_q);
+        dev_free(b->d_q);
         b->d_q = nullptr;
         b->q_cap = 0;
         TRY_CUDA(dev_malloc(&b->d_q, sizeof(BatchQuery) * (size_t)n));
@@ -407,7 +407,7 @@ int trav_batch_create(trav_graph *const *graphs, int32_t n, trav_batch **out)
     b->wmax = (b->vmax + 31) / 32;
     b->chunk_cap = (int64_t)b->vmax + b->emax / kMinItem + 1;
     cudaError_t e = cudaSetDevice(b->device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = stream_get(&b->st);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
     if (e == cudaSuccess) e = dev_malloc(&b->d_next, sizeof(unsigned));
@@ -424,19 +424,19 @@ void trav_batch_free(trav_batch *b)
     if (!b) return;
     cudaSetDevice(b->device);
     if (b->st) cudaStreamSynchronize(b->st);
-    cudaFree(b->team_mem);
-    cudaFree(b->d_teams);
-    cudaFree(b->ctl);
-    cudaFree(b->d_q);
-    cudaFree(b->d_next);
+    dev_free(b->team_mem);
+    dev_free(b->d_teams);
+    dev_free(b->ctl);
+    dev_free(b->d_q);
+    dev_free(b->d_next);
     for (auto &kv : b->light) light_rows_free(&kv.second);
     if (b->cst) cudaStreamSynchronize(b->cst);
-    cudaFree(b->staging);
+    dev_free(b->staging);
     cudaFreeHost(b->done);
-    if (b->cst) cudaStreamDestroy(b->cst);
+    stream_put(b->cst);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
-    if (b->st) cudaStreamDestroy(b->st);
+    stream_put(b->st);
     delete b;
 }
 
@@ -471,7 +471,7 @@ int trav_batch_run_host(trav_batch *b, const trav_query *queries, int32_t n, int
         at[(size_t)i + 1] = at[(size_t)i] + 4 * (size_t)b->graphs[(size_t)queries[i].graph]->g.V;
     if (at[(size_t)n] > b->staging_bytes) {
         if (b->cst) TRY_CUDA(cudaStreamSynchronize(b->cst));
-        cudaFree(b->staging);
+        dev_free(b->staging);
         b->staging = nullptr;
         b->staging_bytes = 0;
         // Team scratch is sized to the free memory when it is allocated, so on
@@ -481,7 +481,7 @@ int trav_batch_run_host(trav_batch *b, const trav_query *queries, int32_t n, int
         TRY_CUDA(dev_malloc(&b->staging, at[(size_t)n]));
         b->staging_bytes = at[(size_t)n];
     }
-    if (!b->cst) TRY_CUDA(cudaStreamCreateWithFlags(&b->cst, cudaStreamNonBlocking));
+    if (!b->cst) TRY_CUDA(stream_get(&b->cst));
     if (n > b->done_cap) {
         cudaFreeHost(b->done);
         b->done = nullptr;

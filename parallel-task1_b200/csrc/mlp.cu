@@ -169,15 +169,15 @@ struct MlpDev {
     int *y = nullptr;
     ~MlpDev()
     {
-        cudaFree(p);
-        cudaFree(g);
-        cudaFree(m);
-        cudaFree(v);
-        cudaFree(x);
-        cudaFree(partial);
-        cudaFree(lpart);
-        cudaFree(loss);
-        cudaFree(y);
+        dev_free(p);
+        dev_free(g);
+        dev_free(m);
+        dev_free(v);
+        dev_free(x);
+        dev_free(partial);
+        dev_free(lpart);
+        dev_free(loss);
+        dev_free(y);
     }
 };
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string>
+#include <vector>
 
 #include "../../include/trav.h"
 
@@ -88,6 +89,7 @@ struct Ctl {
 
 // Device graph: int32 CSR over relabelled ids + transposed CSR.
 struct DevGraph {
+    void *mem = nullptr;          // the allocation behind the arrays
     int32_t V = 0;
     int64_t E = 0;
     int32_t max_out_degree = 0;
@@ -115,6 +117,7 @@ struct LightRows {
 
 // Per-handle traversal workspace (scratch memory of the persistent kernels).
 struct Workspace {
+    void *mem = nullptr;          // the allocation behind the scratch arrays (not ctl, the plans and the light rows)
     int32_t V = 0;
     int64_t chunk_cap = 0;
     // V 64-bit words: BFS levels (int32, the first V words) or SSSP distance
@@ -260,15 +263,58 @@ int cuda_fail(cudaError_t e, const char *what);
 // the kernels may dereference); false for host memory and unknown pointers.
 bool is_device_ptr(const void *p);
 
-// Every device allocation of the library goes through dev_malloc: cudaMalloc,
-// unless a test armed trav_inject_alloc_failure, in which case the armed
+// Every device allocation of the library goes through dev_malloc and back
+// through dev_free (device_memory.cu), which keeps freed blocks for the next
+// call, up to a bound.  When a test armed trav_inject_alloc_failure, the armed
 // allocation fails with cudaErrorMemoryAllocation as cudaMalloc would.
 cudaError_t dev_malloc_bytes(void **p, size_t bytes);
+void dev_free(void *p);
+// True when the armed failure falls on this allocation (each array of a DevSlab counts as one).
+bool alloc_failure_due();
+void arm_alloc_failure(int32_t after);
+// A non-blocking stream of the current device, and back once its work has finished.
+cudaError_t stream_get(cudaStream_t *st);
+void stream_put(cudaStream_t st);
 template <class T>
 inline cudaError_t dev_malloc(T **p, size_t bytes)
 {
     return dev_malloc_bytes(reinterpret_cast<void **>(p), bytes);
 }
+
+// Several arrays in one allocation: add() each, then commit().  The slab owns
+// the memory until release() hands it on (to be freed with dev_free).
+class DevSlab {
+public:
+    ~DevSlab() { dev_free(mem_); }
+    template <class T>
+    void add(T **p, int64_t n)
+    {
+        *p = nullptr;
+        parts_.push_back(Part{reinterpret_cast<void **>(p), bytes_});
+        bytes_ += (sizeof(T) * (size_t)(n > 0 ? n : 1) + 255) & ~(size_t)255;
+    }
+    cudaError_t commit()
+    {
+        for (size_t i = 0; i + 1 < parts_.size(); i++)
+            if (alloc_failure_due()) return cudaErrorMemoryAllocation;
+        const cudaError_t e = dev_malloc_bytes(&mem_, bytes_);
+        if (e != cudaSuccess) return e;
+        for (const Part &p : parts_) *p.at = static_cast<unsigned char *>(mem_) + p.offset;
+        return cudaSuccess;
+    }
+    void *release()
+    {
+        void *m = mem_;
+        mem_ = nullptr;
+        return m;
+    }
+
+private:
+    struct Part { void **at; size_t offset; };
+    std::vector<Part> parts_;
+    size_t bytes_ = 0;
+    void *mem_ = nullptr;
+};
 
 // ingest.cu
 int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_dst, const float *d_w,

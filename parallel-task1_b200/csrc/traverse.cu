@@ -2113,9 +2113,9 @@ int count_light(const DevGraph &g, float delta, int32_t *nlight, cudaStream_t st
 
 void light_rows_free(LightRows *lr)
 {
-    cudaFree(lr->nlight);
-    cudaFree(lr->loff);
-    cudaFree(lr->ledge);
+    dev_free(lr->nlight);
+    dev_free(lr->loff);
+    dev_free(lr->ledge);
     *lr = LightRows{};
 }
 
@@ -2142,7 +2142,7 @@ int light_rows_build(const DevGraph &g, float delta, LightRows *lr, cudaStream_t
     if (e == cudaSuccess && g.V > 0) e = cudaMemcpyAsync(&last[0], lr->loff + g.V - 1, 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && g.V > 0) e = cudaMemcpyAsync(&last[1], lr->nlight + g.V - 1, 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(tmp);
+    dev_free(tmp);
     if (e != cudaSuccess) return cuda_fail(e, "light row offsets");
     const int32_t total = last[0] + last[1];
     TRY_CUDA(cudaMemcpyAsync(lr->loff + g.V, &total, sizeof(int32_t), cudaMemcpyHostToDevice, st));
@@ -2184,7 +2184,7 @@ int workspace_ensure(Workspace *ws, const DevGraph &g, int nqueries, cudaStream_
     if (ws->ctl && ws->V == g.V) {
         if (nqueries <= ws->ctl_cap) return TRAV_OK;
         TRY_CUDA(cudaStreamSynchronize(st));
-        cudaFree(ws->ctl);
+        dev_free(ws->ctl);
         ws->ctl = nullptr;
         ws->ctl_cap = 0;
         TRY_CUDA(dev_malloc(&ws->ctl, sizeof(Ctl) * (size_t)nqueries));
@@ -2196,22 +2196,22 @@ int workspace_ensure(Workspace *ws, const DevGraph &g, int nqueries, cudaStream_
     const int64_t W = (V + 31) / 32;
     ws->V = g.V;
     ws->chunk_cap = V + g.E / kMinItem + 1;
-    TRY_CUDA(dev_malloc(&ws->value, sizeof(unsigned long long) * V));
-    TRY_CUDA(dev_malloc(&ws->rcls, sizeof(unsigned char) * V));
-
-    TRY_CUDA(dev_malloc(&ws->visited, sizeof(unsigned) * W));
-    TRY_CUDA(dev_malloc(&ws->front[0], sizeof(unsigned) * W));
-    TRY_CUDA(dev_malloc(&ws->front[1], sizeof(unsigned) * W));
+    DevSlab mem;
+    unsigned long long *words = nullptr;
+    mem.add(&words, V);
+    mem.add(&ws->rcls, V);
+    mem.add(&ws->visited, W);
     for (int i = 0; i < 2; i++) {
-        TRY_CUDA(dev_malloc(&ws->queue[i], sizeof(int32_t) * V));
-        TRY_CUDA(dev_malloc(&ws->far[i], sizeof(int32_t) * V));
+        mem.add(&ws->front[i], W);
+        mem.add(&ws->queue[i], V);
+        mem.add(&ws->far[i], V);
+        mem.add(&ws->hq[i], V);
+        mem.add(&ws->chunks[i], ws->chunk_cap);
+        mem.add(&ws->hchunks[i], ws->chunk_cap);
     }
-    for (int i = 0; i < 2; i++) {
-        TRY_CUDA(dev_malloc(&ws->hq[i], sizeof(int32_t) * V));
-        TRY_CUDA(dev_malloc(&ws->hchunks[i], sizeof(int2) * ws->chunk_cap));
-    }
-    TRY_CUDA(dev_malloc(&ws->chunks[0], sizeof(int2) * ws->chunk_cap));
-    TRY_CUDA(dev_malloc(&ws->chunks[1], sizeof(int2) * ws->chunk_cap));
+    TRY_CUDA(mem.commit());
+    ws->value = reinterpret_cast<unsigned *>(words);
+    ws->mem = mem.release();
     TRY_CUDA(dev_malloc(&ws->ctl, sizeof(Ctl) * (size_t)nqueries));
     ws->ctl_cap = nqueries;
     return TRAV_OK;
@@ -2219,25 +2219,11 @@ int workspace_ensure(Workspace *ws, const DevGraph &g, int nqueries, cudaStream_
 
 void workspace_free(Workspace *ws)
 {
-    cudaFree(ws->value);
-    cudaFree(ws->rcls);
-    cudaFree(ws->visited);
-    cudaFree(ws->front[0]);
-    cudaFree(ws->front[1]);
-    for (int i = 0; i < 2; i++) {
-        cudaFree(ws->queue[i]);
-        cudaFree(ws->far[i]);
-    }
+    dev_free(ws->mem);
     light_rows_free(&ws->light);
-    for (int i = 0; i < 2; i++) {
-        cudaFree(ws->hq[i]);
-        cudaFree(ws->hchunks[i]);
-    }
-    cudaFree(ws->chunks[0]);
-    cudaFree(ws->chunks[1]);
-    cudaFree(ws->ctl);
-    cudaFree(ws->plan[0]);
-    cudaFree(ws->plan[1]);
+    dev_free(ws->ctl);
+    dev_free(ws->plan[0]);
+    dev_free(ws->plan[1]);
     *ws = Workspace{};
 }
 
@@ -2366,7 +2352,7 @@ int query_bytes(const DevGraph &g, Workspace *ws, int q, int kind, int64_t *byte
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(acc);
+    dev_free(acc);
     if (e != cudaSuccess) return cuda_fail(e, "query_bytes");
     *reached = (int64_t)h[0];
     *reached_edges = (int64_t)h[1];
