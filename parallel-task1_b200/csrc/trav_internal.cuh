@@ -68,6 +68,19 @@ struct Ctl {
     int nphase;                   // phases logged below
     int ndec;                     // schedule decisions logged below
     int cur_query;                // batch launches: the query the team runs next
+    // state of a query that the narrow kernel hands over to the wide one (see narrow.cuh)
+    struct Rows {
+        unsigned q, chunks, big;  // short rows, chunk items, and the rows they come from
+    };
+    struct Resume {
+        int active;               // the wide kernel goes on (0: the query is over)
+        int wrote;                // and its results are written back
+        Rows frontier, heavy;
+        unsigned long long nf, mf, mu, nf_prev, scanned;
+        int steps, buckets, fcur, min_far;
+        unsigned far_len, round, h_start, f_start;
+        float thr, lo;
+    } resume;
     unsigned char dirs[kMaxTrace];       // BFS: direction of step s (0 top-down, 1 bottom-up)
     unsigned int frontier[kMaxTrace];    // BFS: frontier size of step s; SSSP: of expansion s
     // phase log (CTA 0, after each grid barrier): kind (0 top-down, 1 bottom-up,

@@ -19,6 +19,7 @@
 #include <climits>
 #include <cmath>
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <mutex>
 
@@ -1215,6 +1216,8 @@ __device__ __forceinline__ void init_counters(CtaCounters &cc)
     __syncthreads();
 }
 
+#include "narrow.cuh"
+
 // --------------------------------------------------------------- BFS kernel
 // Shared memory of one query's CTA (the bodies below run inside the
 // single-query kernels and inside the batch kernel).
@@ -1237,7 +1240,10 @@ __device__ __forceinline__ void load_mlp(const TravArgs &a, QueryShared &sh, int
 
 // One query on the CTAs [a.cta0, a.cta0 + a.ctas), starting at phase ph0 of the
 // counter-slot ring.  Returns the next phase index, or -1 when the query failed
-// (the error is in a.ctl->err).
+// (the error is in a.ctl->err).  kResume: go on from ctl->resume, after the narrow
+// kernel (a kernel of its own, because the registers that the two beginnings
+// take together spill in the rounds: 5-9% on a query).
+template <bool kResume>
 __device__ __forceinline__ int bfs_query(const TravArgs &a, QueryShared &sh, int ph0)
 {
     SlotView &s_view = sh.view;
@@ -1255,29 +1261,51 @@ __device__ __forceinline__ int bfs_query(const TravArgs &a, QueryShared &sh, int
 
     load_mlp(a, sh, mlp_param_count(kBfsOut));
     init_counters(cc);
-    for (int v = gtid; v < a.V; v += nth) reinterpret_cast<int *>(a.value)[v] = v == s ? 0 : -1;
-    if (!a.color) {
-        for (int w = gtid; w < a.W; w += nth) a.visited[w] = w == (s >> 5) ? 1u << (s & 31) : 0u;
-    } else {
-        // vertex mask: vertices of another color start out visited, so no
-        // step (top-down or bottom-up) ever reaches them; their levels stay -1
-        for (unsigned w = gwarp; w < (unsigned)a.W; w += nwarps) {
-            const int v = (int)(w * 32 + lane_id());
-            const bool pre = v < a.V && (v == s || __ldg(&a.color[v]) != a.color_want);
-            const unsigned m = __ballot_sync(kFull, pre);
-            if (lane_id() == 0) a.visited[w] = m;
-        }
-    }
     unsigned nq, nch;
-    seed_part(a, s, __ldg(&a.out_off[s]), __ldg(&a.out_off[s + 1]), a.q0, a.chunks0, nq, nch);
-    clear_ahead(a, ph);
-    if (!grid_sync(a, ph)) return -1;
-    ph++;
-    if (gtid == 0) ctl->t0_ns = globaltimer();
-
-    const unsigned long long deg_s = (unsigned long long)(__ldg(&a.out_off[s + 1]) - __ldg(&a.out_off[s]));
-    unsigned long long nf = 1, nf_prev = 0, mf = deg_s, mu = (unsigned long long)a.E - deg_s;
+    unsigned long long nf = 1, nf_prev = 0, mf, mu;
     int dir = 0, prev_dir = 0, L = 0, cur = 0, fcur = 0, bu_steps = 0;
+    if constexpr (kResume) {
+        // the narrow kernel ran the first steps (all of them top-down)
+        const Ctl::Resume &r = ctl->resume;
+        if (!r.active) {
+            if (!r.wrote) write_back(a);
+            return ph;
+        }
+        nq = r.frontier.q;
+        nch = r.frontier.chunks;
+        nf = r.nf;
+        nf_prev = r.nf_prev;
+        mf = r.mf;
+        mu = r.mu;
+        L = r.steps;
+        lg.nphase = ctl->nphase;
+        lg.ndec = ctl->ndec;
+        lg.scanned = r.scanned;
+        // every CTA has read the log counters before the leader moves them on
+        if (!grid_sync(a, ph)) return -1;
+        ph++;
+    } else {
+        for (int v = gtid; v < a.V; v += nth) reinterpret_cast<int *>(a.value)[v] = v == s ? 0 : -1;
+        if (!a.color) {
+            for (int w = gtid; w < a.W; w += nth) a.visited[w] = w == (s >> 5) ? 1u << (s & 31) : 0u;
+        } else {
+            // vertex mask: vertices of another color start out visited, so no
+            // step (top-down or bottom-up) ever reaches them; their levels stay -1
+            for (unsigned w = gwarp; w < (unsigned)a.W; w += nwarps) {
+                const int v = (int)(w * 32 + lane_id());
+                const bool pre = v < a.V && (v == s || __ldg(&a.color[v]) != a.color_want);
+                const unsigned m = __ballot_sync(kFull, pre);
+                if (lane_id() == 0) a.visited[w] = m;
+            }
+        }
+        seed_part(a, s, __ldg(&a.out_off[s]), __ldg(&a.out_off[s + 1]), a.q0, a.chunks0, nq, nch);
+        clear_ahead(a, ph);
+        if (!grid_sync(a, ph)) return -1;
+        ph++;
+        if (gtid == 0) ctl->t0_ns = globaltimer();
+        mf = (unsigned long long)(__ldg(&a.out_off[s + 1]) - __ldg(&a.out_off[s]));
+        mu = (unsigned long long)a.E - mf;
+    }
     while (nf > 0) {
         if (L >= a.max_steps) {
             if (gtid == 0) atomicCAS(&ctl->err, 0, kErrBudget);
@@ -1489,10 +1517,11 @@ __device__ __forceinline__ int bfs_query(const TravArgs &a, QueryShared &sh, int
     return ph;
 }
 
+template <bool kResume>
 __global__ void __launch_bounds__(kBlock, TRAV_BFS_MIN_BLOCKS) bfs_persistent(TravArgs a)
 {
     __shared__ QueryShared sh;
-    bfs_query(a, sh, 0);
+    bfs_query<kResume>(a, sh, 0);
 }
 
 // -------------------------------------------------------------- SSSP kernel
@@ -1517,6 +1546,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_BFS_MIN_BLOCKS) bfs_persistent(Tr
 // lowering a distance, so it stamps each vertex it pushes with its own round
 // (an atomicMax that keeps the distance: nothing lowers distances in that
 // phase).
+template <bool kResume>
 __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, DeferStage *defer, int ph0)
 {
     SlotView &s_view = sh.view;
@@ -1544,7 +1574,37 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
     int cur = 0, hcur = 0, fcur = 0;
 
     unsigned h_start = 1, f_start = 1;      // rounds the heavy list / far pile began in
-    if (a.source >= 0) {
+    int steps = 0, buckets = 1;
+    if constexpr (kResume) {
+        // the narrow kernel ran the first phases; round ids go on from its
+        const Ctl::Resume &r = ctl->resume;
+        if (!r.active) {
+            if (!r.wrote) write_back<true>(a);
+            return ph;
+        }
+        nq = r.frontier.q;
+        nch = r.frontier.chunks;
+        nbig = r.frontier.big;
+        hq = r.heavy.q;
+        hch = r.heavy.chunks;
+        hbig = r.heavy.big;
+        far_len = r.far_len;
+        min_far = r.min_far;
+        thr = r.thr;
+        lo = r.lo;
+        fcur = r.fcur;
+        h_start = r.h_start;
+        f_start = r.f_start;
+        steps = r.steps;
+        buckets = r.buckets;
+        lg.nphase = ctl->nphase;
+        lg.ndec = ctl->ndec;
+        lg.scanned = r.scanned;
+        ph = (int)r.round;
+        // every CTA has read the log counters before the leader moves them on
+        if (!grid_sync(a, ph)) return -1;
+        ph++;
+    } else if (a.source >= 0) {
         const int s = a.source;
         for (int v = gtid; v < a.V; v += nth) {
             const unsigned cls = row_class(a, v);
@@ -1594,7 +1654,6 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
         if (gtid == 0) ctl->t0_ns = globaltimer();
     }
 
-    int steps = 0, buckets = 1;
     // Light rounds hold back long light rows whose distance is more than
     // kHoldSlack x delta above the lowest distance of the round's frontier (a
     // vertex at or below that lowest distance is final: every later candidate
@@ -1794,11 +1853,12 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
     return ph;
 }
 
+template <bool kResume>
 __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) sssp_persistent(TravArgs a)
 {
     __shared__ QueryShared sh;
     __shared__ DeferStage defer[kWarps];
-    sssp_query(a, sh, defer, 0);
+    sssp_query<kResume>(a, sh, defer, 0);
 }
 
 // ------------------------------------------------------------ batch kernel
@@ -1890,7 +1950,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) batch_persistent
             a.force_dir = -1;
             a.delta = 0.0f;
             a.out_kind = 0;
-            ph = bfs_query(a, sh, ph);
+            ph = bfs_query<false>(a, sh, ph);
         } else {
             // round stamps are phase indices: the team's whole run must fit them
             a.max_steps = (int32_t)min((long long)4 * q.V + 4096, (long long)(kMaxRounds - 2 - ph));
@@ -1899,7 +1959,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) batch_persistent
             a.mean_w = q.mean_w;
             a.max_deg = q.max_deg;
             a.out_kind = 1;
-            ph = sssp_query(a, sh, defer, ph);
+            ph = sssp_query<false>(a, sh, defer, ph);
         }
         if (ph < 0) return;
         if (b.done) __threadfence_system();  // this thread's results, before the next dispatch barrier
@@ -2039,9 +2099,78 @@ int launch_cooperative(const void *fn, int grid, void **params, cudaStream_t st)
     return TRAV_OK;
 }
 
-// Enqueue one persistent launch: clear its control block, launch
-// cooperatively (all CTAs co-resident, which the grid barrier needs).
-int enqueue_persistent(int kind, TravArgs &args, int ctas, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1)
+// Edges up to which a graph of at most kNarrowRows vertices is left to the
+// narrow kernel alone: above, a phase of most of the edges would take its 16 SMs
+// longer than the whole device with its barriers.
+constexpr int64_t kNarrowAloneEdges = 1 << 18;
+
+// CTAs of the narrow kernel's cluster on the current device: 16 (a
+// non-portable size) where the device can place it, else 8, else 0 (none).
+int narrow_ctas(int kind)
+{
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> known[2][kMaxDevices];  // CTAs + 1
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    const int k = known[kind][dev].load();
+    if (k) return k - 1;
+    const void *fn = kind == 0 ? (const void *)bfs_narrow : (const void *)sssp_narrow;
+    int found = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NarrowShared)) == cudaSuccess &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        for (int c = kNarrowCtas; c >= 8 && !found; c /= 2) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)c);
+            cfg.blockDim = dim3(kNarrowThreads);
+            cfg.dynamicSmemBytes = sizeof(NarrowShared);
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)c;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1) found = c;
+        }
+    }
+    cudaGetLastError();
+    known[kind][dev].store(found + 1);
+    return found;
+}
+
+// The query's initialisation (by the whole device unless the graph is small)
+// and its narrow phases.
+int launch_narrow(int kind, const TravArgs &args, int cluster, int alone, cudaStream_t st)
+{
+    TravArgs a = args;
+    if (a.V > kNarrowOwn) {
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (kind == 0) bfs_init_kernel<<<sms * 8, 256, 0, st>>>(a);
+        else sssp_init_kernel<<<sms * 8, 256, 0, st>>>(a);
+        TRY_CUDA(cudaGetLastError());
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)cluster);
+    cfg.blockDim = dim3(kNarrowThreads);
+    cfg.dynamicSmemBytes = sizeof(NarrowShared);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void *params[] = {&a, &alone};
+    TRY_CUDA(cudaLaunchKernelExC(&cfg, kind == 0 ? (const void *)bfs_narrow : (const void *)sssp_narrow, params));
+    return TRAV_OK;
+}
+
+// Enqueue one query: clear its control block, run its narrow phases if `narrow`,
+// then the persistent kernel cooperatively (all CTAs co-resident, which the grid
+// barrier needs).
+int enqueue_persistent(int kind, TravArgs &args, int ctas, bool narrow, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1)
 {
     int grid = persistent_grid_size(kind);
     if (grid <= 0) return TRAV_ERR_CUDA;
@@ -2050,8 +2179,24 @@ int enqueue_persistent(int kind, TravArgs &args, int ctas, cudaStream_t st, cuda
     args.ctas = grid;
     TRY_CUDA(cudaMemsetAsync(args.ctl, 0, offsetof(Ctl, dirs), st));
     if (ev0) TRY(record_event(ev0, st));
+    int alone = 0;
+    bool resume = false;
+    if (narrow) {
+        const int cluster = narrow_ctas(kind);
+        if (cluster > 0) {
+            // Small graphs run in the narrow kernel alone: no phase of theirs can
+            // outgrow its queues, and the wide launch would only add its 5-8 us.
+            alone = args.V <= kNarrowRows && args.E <= kNarrowAloneEdges;
+            TRY(launch_narrow(kind, args, cluster, alone, st));
+            resume = true;
+        }
+    }
     void *params[] = {&args};
-    TRY(launch_cooperative(kind == 0 ? (const void *)bfs_persistent : (const void *)sssp_persistent, grid, params, st));
+    if (!alone) {
+        const void *fn = kind == 0 ? (resume ? (const void *)bfs_persistent<true> : (const void *)bfs_persistent<false>)
+                                   : (resume ? (const void *)sssp_persistent<true> : (const void *)sssp_persistent<false>);
+        TRY(launch_cooperative(fn, grid, params, st));
+    }
     if (ev1) TRY(record_event(ev1, st));
     return TRAV_OK;
 }
@@ -2077,8 +2222,8 @@ int persistent_grid_size(int kind)
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const void *fn = kind == 0 ? (const void *)bfs_persistent
-                   : kind == 1 ? (const void *)sssp_persistent : (const void *)batch_persistent;
+    const void *fn = kind == 0 ? (const void *)bfs_persistent<false>
+                   : kind == 1 ? (const void *)sssp_persistent<false> : (const void *)batch_persistent;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kBlock, 0);
     if (e != cudaSuccess || per < 1 || sms < 1) {
         cuda_fail(e == cudaSuccess ? cudaErrorInvalidConfiguration : e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
@@ -2268,6 +2413,16 @@ static TravArgs make_args(const DevGraph &g, Workspace *ws)
     return a;
 }
 
+constexpr int kNarrowDegree = 8;  // mean degree up to which an SSSP query begins in the narrow kernel
+
+// Queries that may begin in the narrow kernel: those whose launch shape, step
+// budget, wait limit and decisions are not set by the caller.  (The direction
+// network is consulted in the wide kernel only.)
+static bool narrow_query(const Workspace &ws, int kind)
+{
+    return ws.grid[kind] == 0 && ws.max_steps == 0 && ws.timeout_ns == 0 && ws.plan_len[kind] == 0;
+}
+
 int launch_bfs(const DevGraph &g, Workspace *ws, int q, int32_t source_new, const trav_bfs_opts &o,
                const float *mlp, void *out, int out_kind, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1,
                const int32_t *color, int32_t color_want)
@@ -2289,7 +2444,7 @@ int launch_bfs(const DevGraph &g, Workspace *ws, int q, int32_t source_new, cons
     a.mlp_margin = ws->mlp_margin[0];
     a.plan = ws->plan[0];
     a.plan_len = ws->plan_len[0];
-    return enqueue_persistent(0, a, ws->grid[0], st, ev0, ev1);
+    return enqueue_persistent(0, a, ws->grid[0], narrow_query(*ws, 0) && !mlp, st, ev0, ev1);
 }
 
 int launch_sssp(const DevGraph &g, Workspace *ws, int q, int32_t source_new, float delta, const float *mlp,
@@ -2323,7 +2478,12 @@ int launch_sssp(const DevGraph &g, Workspace *ws, int q, int32_t source_new, flo
     a.mlp_margin = ws->mlp_margin[1];
     a.plan = ws->plan[1];
     a.plan_len = ws->plan_len[1];
-    return enqueue_persistent(1, a, ws->grid[1], st, ev0, ev1);
+    // On denser graphs the second or third round outgrows the narrow kernel, and
+    // handing over the hubs' heavy rows costs more than its rounds saved (RMAT
+    // scale 16, edge factor 16, Bellman-Ford: 5% slower; uniform degree 16: 3%
+    // faster; grid of degree 4: 1.4 times as fast).
+    const bool sparse = g.E <= (int64_t)kNarrowDegree * g.V || g.V <= kNarrowRows;
+    return enqueue_persistent(1, a, ws->grid[1], narrow_query(*ws, 1) && source_new >= 0 && sparse, st, ev0, ev1);
 }
 
 // Byte accounting of query q, which must be the last query run (its results

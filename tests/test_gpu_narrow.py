@@ -1,0 +1,94 @@
+"""Queries that run (or begin) in the narrow kernel, at the sizes where it changes path: rows around a segment and
+around a whole queue, frontiers that outgrow the queue at once, after some phases or never, graphs around the sizes
+that are initialised there and that run there alone.  Levels and distances equal the oracle bit for bit, and the
+logs describe the same traversal."""
+import numpy as np
+import pytest
+
+import oracle as O
+import pytrav as T
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(V, s, d, w, src, deltas=(0.0, 0.3, 40.0)):
+    s, d, w = np.asarray(s, np.int32), np.asarray(d, np.int32), np.asarray(w, np.float32)
+    g = T.Graph.from_edges(V, s, d, w)
+    csr = O.csr(V, s, d, w)
+    want = O.bfs_levels(V, s, d, src, csr_arrays=csr)
+    for force in (-1, 0, 1):
+        assert np.array_equal(g.bfs([src], force_direction=force)[0], want), force
+        st = g.last_stats()
+        dirs, frontier = g.last_bfs_trace()
+        kind = g.last_phase_log()[0]
+        assert st.steps == want.max() + 1
+        n = len(dirs)  # the logs hold at most 4096 entries
+        assert frontier.tolist() == [int((want == i).sum()) for i in range(n)]
+        if len(kind) < 4096:
+            assert [k for k in kind if k in (0, 1)] == dirs.tolist()
+    ref = O.dijkstra(V, s, d, w, src, csr_arrays=csr).view(np.uint32)
+    for delta in deltas:
+        for _ in range(2):
+            assert np.array_equal(g.sssp([src], delta=delta)[0].view(np.uint32), ref), delta
+    g.free()
+
+
+def _grid(h, wd, seed):
+    idx = np.arange(h * wd).reshape(h, wd)
+    p = [(idx[:, :-1], idx[:, 1:]), (idx[:, 1:], idx[:, :-1]), (idx[:-1], idx[1:]), (idx[1:], idx[:-1])]
+    s, d = (np.concatenate([x[k].ravel() for x in p]) for k in (0, 1))
+    return h * wd, s, d, np.random.default_rng(seed).integers(1, 100, len(s)).astype(np.float32)
+
+
+@pytest.mark.parametrize("h,wd", [(1, 3), (64, 96), (64, 97), (5, 3000), (362, 362), (400, 331)])
+def test_grids_stay_narrow(h, wd):
+    _check(*_grid(h, wd, h), src=h * wd // 2)
+
+
+@pytest.mark.parametrize("deg", [0, 1, 127, 128, 129, 640, 6143, 6144, 6145, 20_000])
+def test_rows_at_the_segment_and_queue_limits(deg):
+    """A hub behind a path, with `deg` out-edges to leaves that join again and go on."""
+    V = deg + 8
+    s = [0, 1] + [2] * deg + [3 + i for i in range(deg)] + [V - 3, V - 2]
+    d = [1, 2] + [3 + i for i in range(deg)] + [V - 3] * deg + [V - 2, V - 1]
+    rng = np.random.default_rng(deg)
+    _check(V, s, d, (rng.integers(0, 9, len(s)) / 8).astype(np.float32), 0)
+
+
+@pytest.mark.parametrize("V,E,seed", [(6144, 30_000, 1), (6145, 30_000, 2), (6144, 300_000, 3), (131_072, 400_000, 4),
+                                      (131_073, 400_000, 5), (3000, 262_144, 6), (40_000, 60_000, 7)])
+def test_random_graphs_change_over(V, E, seed):
+    rng = np.random.default_rng(seed)
+    s, d = rng.integers(0, V, E), rng.integers(0, V, E)
+    s[0] = 7
+    _check(V, s, d, rng.random(E, dtype=np.float32), 7, deltas=(0.0, 0.05, 0.5))
+
+
+def test_learned_widths_and_several_sources():
+    V, s, d, w = _grid(150, 170, 3)
+    s, d = s.astype(np.int32), d.astype(np.int32)
+    g = T.Graph.from_edges(V, s, d, w)
+    g.set_mlp(1, np.random.default_rng(1).normal(scale=2.0, size=T.mlp_param_count(1)))
+    srcs = [0, 77, V - 1]
+    got = g.sssp(srcs, delta=3.0, schedule=T.SCHEDULE_LEARNED)
+    x, ch, ph, lo, hi = g.last_decisions()
+    assert len(ch) > 0 and np.all(hi > lo) and np.all(np.diff(lo) > 0) and np.all(np.isfinite(x))
+    for k, src in enumerate(srcs):
+        assert np.array_equal(got[k].view(np.uint32), O.dijkstra(V, s, d, w, src).view(np.uint32))
+    g.free()
+
+
+def test_masked_sweep_through_the_narrow_kernel():
+    """The vertex mask reaches the BFS kernels when the edge-list sweeps give up (a long path)."""
+    import torch
+
+    n = 20_000
+    s = np.arange(n - 1).astype(np.int32)[::-1].copy()
+    d = (s + 1).astype(np.int32)
+    trees = (np.arange(n) >= 15_000).astype(np.int32)
+    vis = torch.full((n,), 9, dtype=torch.uint8, device="cuda")
+    tp = torch.tensor([3], dtype=torch.int32, device="cuda")
+    ts, td, tt = (torch.from_numpy(x).cuda() for x in (s, d, trees))
+    T._check(T.lib().trav_reach_el_masked(ts.data_ptr(), td.data_ptr(), n, n - 1, tp.data_ptr(), tt.data_ptr(),
+                                          vis.data_ptr()))
+    assert np.array_equal(vis.cpu().numpy(), O.reach_masked(n, s, d, 3, trees))
