@@ -133,13 +133,21 @@ struct SlotView {
     unsigned long long scanned;
 };
 
+__shared__ unsigned long long s_target;  // arrivals the last grid barrier waited for (thread 0)
+
+__device__ __forceinline__ void init_barrier()
+{
+    if (threadIdx.x == 0) s_target = 0;
+}
+
 // Grid-wide barrier with a bounded wait.  After the CTA barrier, thread 0 of
-// every CTA adds one to a single arrival counter with an acquire-release
-// atomic (which orders the CTA's writes of the phase before it).  The counter
-// only grows, so barrier k of a launch is passed once it reaches
-// k * gridDim.x: there is no reset and no generation word, and the critical
-// path is one arrival plus one poll.  (A tree of reset counters puts a chain of
-// dependent atomics and fences on that path instead.)  Waiters poll with an
+// every CTA adds one to a single arrival counter with a release (which orders
+// the CTA's writes of the phase before it).  The counter only grows, so barrier
+// k of a launch is passed once it reaches k * CTAs: there is no reset, no
+// generation word and no need of the counter's old value (an atomic with a
+// result takes about 1000 cycles on a B200), and the critical path is one
+// arrival plus one poll.  (A tree of reset counters puts a chain of dependent
+// atomics and fences on that path instead.)  Waiters poll with an
 // acquire load and give up after timeout_ns, or when another CTA already
 // failed; the barrier then returns false in every thread of the CTA.
 //
@@ -156,25 +164,23 @@ __device__ bool grid_sync(const TravArgs &a, int phase, SlotView *view = nullptr
     if (threadIdx.x < 32) {
         if (threadIdx.x == 0) {
             int ok = 1;
-            const unsigned long long nb = (unsigned long long)a.ctas;
-            unsigned long long old;
-            asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(old) : "l"(&ctl->bar_count) : "memory");
-            const unsigned long long target = (old / nb + 1) * nb;
-            if (old + 1 != target) {
-                const unsigned long long t0 = globaltimer();
-                unsigned ns = 32;
-                while (true) {
-                    unsigned long long c;
-                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(&ctl->bar_count) : "memory");
-                    if (c >= target) break;
-                    if (ld_relaxed_int(&ctl->err) != 0) { ok = 0; break; }
-                    __nanosleep(ns);
-                    if (ns < 128) ns <<= 1;
-                    if (globaltimer() - t0 > timeout_ns) {
-                        if (atomicCAS(&ctl->err, 0, kErrTimeout) == 0) atomicExch(&ctl->err_phase, phase);
-                        ok = 0;
-                        break;
-                    }
+            const unsigned long long target = s_target + (unsigned long long)a.ctas;
+            s_target = target;
+            asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
+            const unsigned long long t0 = globaltimer();
+            unsigned ns = 32;
+            for (unsigned i = 0;; i++) {
+                unsigned long long c;
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(&ctl->bar_count) : "memory");
+                if (c >= target) break;
+                __nanosleep(ns);
+                if (ns < 128) ns <<= 1;
+                if (i & 3u) continue;
+                if (ld_relaxed_int(&ctl->err) != 0) { ok = 0; break; }
+                if (globaltimer() - t0 > timeout_ns) {
+                    if (atomicCAS(&ctl->err, 0, kErrTimeout) == 0) atomicExch(&ctl->err_phase, phase);
+                    ok = 0;
+                    break;
                 }
             }
             s_ok = ok;
@@ -569,7 +575,9 @@ struct WarpStage {
     int q[2][kWQ];
     int big[2][kWBig];
     int far[kWFar];
-    int tu[32], trb[32], tpre[32];  // the current warp tile
+    // rows of the current warp tile: vertex, first edge less the edges of the rows
+    // before, distance
+    int tu[32], trb[32];
     float tdu[32];
 };
 
@@ -741,11 +749,22 @@ __device__ __forceinline__ void push_far(Pusher &p, bool flag, int v, int key)
 // the counters and publishes them with one atomic each.  CTA-collective.
 __device__ void finish_phase(Pusher &p, CtaCounters &cc)
 {
-    for (int t = 0; t < 2; t++) {
-        if (p.nq[t]) flush_q(p, t);
+    for (int t = 0; t < 2; t++)
         if (p.nbig[t]) flush_big(p, t);
+    __syncwarp();
+    if (p.nq[0] | p.nq[1] | p.nfar) {
+        // one round trip for the three reservations
+        const unsigned lane = lane_id(), n = lane == 0 ? p.nq[0] : lane == 1 ? p.nq[1] : lane == 2 ? p.nfar : 0u;
+        unsigned base = lane == 0 ? p.o->qbase[0] : lane == 1 ? p.o->qbase[1] : p.o->fbase;
+        Slot *sl = p.o->slot;
+        if (n) base += atomicAdd(lane == 0 ? &sl->q_add : lane == 1 ? &sl->hq_add : &sl->far_add, n);
+        const unsigned b0 = __shfl_sync(kFull, base, 0), b1 = __shfl_sync(kFull, base, 1), bf = __shfl_sync(kFull, base, 2);
+        for (unsigned i = lane; i < p.nq[0]; i += 32) p.o->q[0][b0 + i] = p.s->q[0][i];
+        for (unsigned i = lane; i < p.nq[1]; i += 32) p.o->q[1][b1 + i] = p.s->q[1][i];
+        for (unsigned i = lane; i < p.nfar; i += 32) p.o->farp[bf + i] = p.s->far[i];
+        p.nq[0] = p.nq[1] = p.nfar = 0;
+        __syncwarp();
     }
-    if (p.nfar) flush_far(p);
     const unsigned long long mf = __reduce_add_sync(kFull, (unsigned)p.mf);  // per-lane parts fit 32 bits
     unsigned long long sc = p.scanned;
 #pragma unroll
@@ -781,8 +800,14 @@ __device__ void finish_phase(Pusher &p, CtaCounters &cc)
 }
 
 // Expand a frontier (part kPart of each row) in one phase: chunk items one
-// warp each, then the short-row queue in 32-vertex warp tiles (edge-balanced
-// within the tile).  Every lane carries kBatch independent edges per round so
+// warp each, then the short-row queue in warp tiles (edge-balanced within the
+// tile).  A phase with little work is a chain of dependent loads and atomics,
+// so its work is cut smaller and spread wider: tiles and items shrink with the
+// work per warp, and consecutive ones go to different CTAs.  Measured on a B200
+// (kernel time): uniform 1 M vertices of degree 16, BFS 193 -> 148 us, SSSP 1425
+// -> 1090 us; Bellman-Ford on RMAT scale 16 382 -> 330 us (three sources); 512
+// queries on 64 small graphs 4.89 -> 4.63 ms; RMAT scale 21, 32 queries 8.15 ->
+// 7.66 ms.  Every lane carries kBatch independent edges per round so
 // their loads and atomics overlap.
 template <int kPart, class Vis>
 __device__ void expand_frontier(const TravArgs &a, const int32_t *q, unsigned nq, const int2 *chunks, unsigned nch,
@@ -790,12 +815,19 @@ __device__ void expand_frontier(const TravArgs &a, const int32_t *q, unsigned nq
 {
     constexpr int kBatch = Vis::kBatch;
     const int lane = (int)lane_id();
-    const unsigned gwarp = (unsigned)team_tid(a) >> 5, nwarps = (unsigned)team_threads(a) >> 5;
-    for (unsigned c = gwarp; c < nch; c += nwarps) {
-        const int2 it = chunks[c];
-        const int u = it.x, start = it.y;
+    // consecutive units go to different CTAs, so that few of them spread over the SMs
+    const unsigned nwarps = (unsigned)team_threads(a) >> 5;
+    const unsigned gwarp = (threadIdx.x >> 5) * (unsigned)a.ctas + (blockIdx.x - (unsigned)a.cta0);
+    // With fewer items than warps, several warps share an item (at least 64 edges each).
+    int is = 0;
+    while (is < 3 && nch <= nwarps >> (is + 1) && a.item >> (is + 1) >= 64) is++;
+    const int sub_len = (a.item + (1 << is) - 1) >> is;
+    for (unsigned c = gwarp; c < nch << is; c += nwarps) {
+        const int2 it = chunks[c >> is];
+        const int u = it.x, start = it.y + (int)(c & ((1u << is) - 1u)) * sub_len;
         const int2 rp = row_part(a, u, kPart);
-        const int end = min(start + a.item, rp.y);
+        const int end = min(min(start + sub_len, it.y + a.item), rp.y);
+        if (start >= end) continue;
         const float du = vis.begin(u);
         if (kHoldSlack >= 0.0f && kPart == kPartLight && nq > 0 && vis.hold(du)) {
             // A long light row (a hub's) whose distance is well above the
@@ -823,10 +855,16 @@ __device__ void expand_frontier(const TravArgs &a, const int32_t *q, unsigned nq
         }
     }
     WarpStage *s = p.s;
-    for (unsigned t0 = gwarp * 32; t0 < nq; t0 += nwarps * 32) {
+    // A phase with fewer short rows than 32 per warp spreads them over more
+    // warps, down to 4 a tile: the rounds of a tile are a serial chain.
+    int ts = 5;
+    while (ts > 2 && nq <= nwarps << (ts - 1)) ts--;
+    // the first tiles go to the warps after those with the last items
+    const unsigned past = (nch << is) % nwarps, first = gwarp >= past ? gwarp - past : gwarp + nwarps - past;
+    for (unsigned t0 = first << ts; t0 < nq; t0 += nwarps << ts) {
         const unsigned i = t0 + lane;
         int u = 0, rb = 0, deg = 0;
-        if (i < nq) {
+        if (lane < 1 << ts && i < nq) {
             u = q[i];
             const int2 pr = row_part(a, u, kPart);
             rb = pr.x;
@@ -839,33 +877,32 @@ __device__ void expand_frontier(const TravArgs &a, const int32_t *q, unsigned nq
             if (lane >= d) incl += y;
         }
         const int total = __shfl_sync(kFull, incl, 31);
-        s->tu[lane] = u;
-        s->trb[lane] = rb;
-        s->tpre[lane] = incl - deg;
-        s->tdu[lane] = deg > 0 ? vis.begin(u) : 0.0f;
+        const int pre = incl - deg;
+        const bool has = deg > 0;
+        const int at = __popc(__ballot_sync(kFull, has) & lanemask_lt());
+        if (has) {
+            s->tu[at] = u;
+            s->trb[at] = rb - pre;
+            s->tdu[at] = vis.begin(u);
+        }
         __syncwarp();
         if (lane == 0) p.scanned += (unsigned long long)total;
-        const int n = (int)min(32u, nq - t0);
         for (int base = 0; base < total; base += 32 * kBatch) {
             int us[kBatch], e[kBatch];
             float ds[kBatch];
             bool ok[kBatch];
 #pragma unroll
             for (int j = 0; j < kBatch; j++) {
-                const int k = base + lane + 32 * j;
+                // lane k of batch j takes edge base + 32 j + k; its row: the rows that
+                // start before the batch, and those that start in it up to k
+                const int b = base + 32 * j, d = pre - b, k = b + lane;
+                const unsigned starts = __reduce_or_sync(kFull, has && (unsigned)d < 32u ? 1u << d : 0u);
+                const unsigned before = (unsigned)__popc(__ballot_sync(kFull, has && d < 0));
+                const int r = (int)(before + __popc(starts & (lanemask_lt() << 1 | 1u))) - 1;
                 ok[j] = k < total;
-                int lo = 0;
-                if (ok[j]) {
-                    int hi = n;
-                    while (hi - lo > 1) {
-                        const int mid = (lo + hi) >> 1;
-                        if (s->tpre[mid] <= k) lo = mid;
-                        else hi = mid;
-                    }
-                }
-                e[j] = s->trb[lo] + (k - s->tpre[lo]);
-                us[j] = s->tu[lo];
-                ds[j] = s->tdu[lo];
+                e[j] = s->trb[r] + k;
+                us[j] = s->tu[r];
+                ds[j] = s->tdu[r];
             }
             vis.template visit_batch<kPart>(us, ds, e, ok, p);
         }
@@ -1521,6 +1558,7 @@ template <bool kResume>
 __global__ void __launch_bounds__(kBlock, TRAV_BFS_MIN_BLOCKS) bfs_persistent(TravArgs a)
 {
     __shared__ QueryShared sh;
+    init_barrier();
     bfs_query<kResume>(a, sh, 0);
 }
 
@@ -1858,6 +1896,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) sssp_persistent(
 {
     __shared__ QueryShared sh;
     __shared__ DeferStage defer[kWarps];
+    init_barrier();
     sssp_query<kResume>(a, sh, defer, 0);
 }
 
@@ -1873,6 +1912,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) batch_persistent
 {
     __shared__ QueryShared sh;
     __shared__ DeferStage defer[kWarps];  // used by the SSSP queries
+    init_barrier();
     const int team = (int)blockIdx.x / b.team_ctas;
     const TeamWs w = b.teams[team];
     TravArgs t{};
@@ -2567,6 +2607,7 @@ __global__ void noalloc_validate_csr(const int32_t *__restrict__ off, const int3
 __global__ void __launch_bounds__(kBlock) bfs_csr_noalloc_kernel(TravArgs a, int32_t *levels)
 {
     __shared__ TileShared ts;
+    init_barrier();
     Ctl *ctl = a.ctl;
     const int gtid = blockIdx.x * kBlock + threadIdx.x, nth = gridDim.x * kBlock;
     const int s = a.source;
