@@ -157,6 +157,7 @@ __device__ __forceinline__ NarrowTotal narrow_totals(int ring, int opened)
     const unsigned lane = threadIdx.x & 31u, C = cluster_size();
     NarrowCount c{};
     if (lane < C) c = on_rank(&s, lane)->cnt[ring];
+    c.segs = min(c.segs, (unsigned)kNarrowSegs);
     NarrowTotal t;
     t.rank = c;
     t.far_len = *reinterpret_cast<volatile unsigned *>(&on_rank(&s, 0)->nfar[opened % 3]);
@@ -208,8 +209,11 @@ __device__ __forceinline__ void narrow_push_row(int out, NarrowCount &c, int v, 
     const unsigned i = atomicAdd(&c.rows, 1u);
     if (len > kNarrowSeg && len <= kNarrowRows) {
         // A long row in few lanes would be a long chain: its segments are units
-        // of their own.  Where they do not fit, the phase has far more edges
-        // than a narrow one may, and the row stays whole.
+        // of their own.  Where they do not fit, the row stays whole: the first
+        // such row fills the segments' places left with empty ones, and none
+        // after it finds room (narrow_totals counts no more than the places).
+        // That takes more than 64k edges in one CTA's queue, which only a graph
+        // that runs here alone goes on with.
         const int more = (len - 1) / kNarrowSeg;
         unsigned at = atomicAdd(&c.segs, (unsigned)more);
         if (at + (unsigned)more <= (unsigned)kNarrowSegs) {
@@ -220,6 +224,12 @@ __device__ __forceinline__ void narrow_push_row(int out, NarrowCount &c, int v, 
                 s.len[out][at] = min(kNarrowSeg, len - k * kNarrowSeg);
             }
             len = kNarrowSeg;
+        } else {
+            for (; at < (unsigned)kNarrowSegs; at++) {
+                s.v[out][kNarrowRows + at] = v;
+                s.begin[out][kNarrowRows + at] = begin;
+                s.len[out][kNarrowRows + at] = 0;
+            }
         }
     }
     s.v[out][i] = v;

@@ -92,3 +92,15 @@ def test_masked_sweep_through_the_narrow_kernel():
     T._check(T.lib().trav_reach_el_masked(ts.data_ptr(), td.data_ptr(), n, n - 1, tp.data_ptr(), tt.data_ptr(),
                                           vis.data_ptr()))
     assert np.array_equal(vis.cpu().numpy(), O.reach_masked(n, s, d, 3, trees))
+
+
+@pytest.mark.parametrize("first,fan", [(127, 1980), (100, 2500), (60, 4000), (20, 6000), (3, 40_000)])
+def test_long_rows_beyond_the_segments_of_a_queue(first, fan):
+    # a small graph whose source has one short row, so that one block of the cluster finds all the long rows of the
+    # next frontier: their segments outnumber the places of its queue
+    V = 1200
+    rng = np.random.default_rng(first)
+    s = np.concatenate([np.zeros(first, np.int64), np.repeat(np.arange(1, first + 1), fan)])
+    d = np.concatenate([np.arange(1, first + 1), rng.integers(0, V, first * fan)])
+    assert len(s) <= 1 << 18
+    _check(V, s, d, rng.uniform(0.01, 1.0, len(s)), 0, deltas=(0.0, 0.3))
