@@ -295,7 +295,7 @@ int run_launch(trav_batch *b, int32_t n, const trav_batch_shape &s, float *ms, u
         teams = (int)std::min<size_t>((size_t)teams, fit);
     }
     TRY(ensure_teams(b, teams));
-    for (int t = 0; t < teams; t++) TRY_CUDA(cudaMemsetAsync(b->ctl + t, 0, offsetof(Ctl, dirs), b->st));
+    TRY_CUDA(cudaMemset2DAsync(b->ctl, sizeof(Ctl), 0, offsetof(Ctl, dirs), (size_t)teams, b->st));
     BatchArgs a{};
     a.queries = b->d_q;
     a.nq = n;
@@ -317,8 +317,7 @@ int run_launch(trav_batch *b, int32_t n, const trav_batch_shape &s, float *ms, u
             std::this_thread::yield();
         }
     }
-    TRY_CUDA(cudaStreamSynchronize(b->st));
-    TRY(check_ctls(b->ctl, teams, "batch"));
+    TRY(check_ctls(b->ctl, teams, "batch", b->st));
     if (prc != TRAV_OK && prc != kBusy) return prc;
     float t = 0.0f;
     TRY_CUDA(cudaEventElapsedTime(&t, b->ev0, b->ev1));

@@ -238,11 +238,11 @@ int run_batch(trav_graph *g, int kind, const int32_t *sources, int32_t n, const 
     } else {
         TRY(enqueue());
     }
-    TRY_CUDA(cudaStreamSynchronize(g->st));
+    const int rc = check_queries(&g->ws, n, kind == 0 ? "bfs" : "sssp", g->st);
     TRY_CUDA(cudaStreamSynchronize(g->cst));
     g->last_kind = kind;
     g->last_n = n;
-    TRY(check_queries(&g->ws, n, kind == 0 ? "bfs" : "sssp"));
+    TRY(rc);
     g->batch_ms.assign((size_t)n, 0.0f);
     for (int32_t q = 0; q < n; q++) TRY_CUDA(cudaEventElapsedTime(&g->batch_ms[(size_t)q], g->ev[2 * q], g->ev[2 * q + 1]));
     return TRAV_OK;
@@ -766,8 +766,7 @@ int trav_bellman_ford_el_f32(const int32_t *src, const int32_t *dst, const float
         reinterpret_cast<unsigned *>(h->ws.queue[1]), d, h->g.old_of_new, vertices);
     TRY_CUDA(cudaGetLastError());
     TRY(launch_sssp(h->g, &h->ws, 0, -1, INFINITY, nullptr, d, 1, h->st, nullptr, nullptr));
-    TRY_CUDA(cudaStreamSynchronize(h->st));
-    return check_queries(&h->ws, 1, "bellman_ford_wrapper");
+    return check_queries(&h->ws, 1, "bellman_ford_wrapper", h->st);
 }
 
 int trav_bfs_el(const int32_t *src, const int32_t *dst, int32_t vertices, int64_t edges, uint8_t *visited,
@@ -797,8 +796,7 @@ int trav_bfs_el(const int32_t *src, const int32_t *dst, int32_t vertices, int64_
     int32_t s_new = 0;
     TRY_CUDA(cudaMemcpy(&s_new, h->g.new_of_old + source, sizeof(int32_t), cudaMemcpyDeviceToHost));
     TRY(launch_bfs(h->g, &h->ws, 0, s_new, o, nullptr, visited, 2, h->st, nullptr, nullptr));
-    TRY_CUDA(cudaStreamSynchronize(h->st));
-    return check_queries(&h->ws, 1, "bfs_wrapper");
+    return check_queries(&h->ws, 1, "bfs_wrapper", h->st);
 }
 
 static __global__ void permute_color_kernel(int32_t *color_new, const int32_t *color, const int32_t *old_of_new,
@@ -845,8 +843,7 @@ int trav_reach_el_masked(const int32_t *src, const int32_t *dst, int32_t vertice
     int32_t p_new = 0;
     TRY_CUDA(cudaMemcpy(&p_new, h->g.new_of_old + p, sizeof(int32_t), cudaMemcpyDeviceToHost));
     TRY(launch_bfs(h->g, &h->ws, 0, p_new, o, nullptr, visited, 2, h->st, nullptr, nullptr, color.p, want));
-    TRY_CUDA(cudaStreamSynchronize(h->st));
-    return check_queries(&h->ws, 1, "trav_reach_el_masked");
+    return check_queries(&h->ws, 1, "trav_reach_el_masked", h->st);
 }
 
 // ----------------------------------------------------------- graph files

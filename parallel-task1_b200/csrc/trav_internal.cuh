@@ -363,9 +363,9 @@ int launch_bfs(const DevGraph &g, Workspace *ws, int q, int32_t source_new, cons
                const int32_t *color = nullptr, int32_t color_want = 0);
 int launch_sssp(const DevGraph &g, Workspace *ws, int q, int32_t source_new, float delta, const float *mlp,
                 void *out, int out_kind, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1);
-// After the stream finished: turn the device status of queries [0, n) into a return code.
-int check_queries(Workspace *ws, int n, const char *what);
-int check_ctls(const Ctl *ctl, int n, const char *what);  // the same for n device control blocks
+// Wait for st and turn the device status of queries [0, n) into a return code.
+int check_queries(Workspace *ws, int n, const char *what, cudaStream_t st);
+int check_ctls(const Ctl *ctl, int n, const char *what, cudaStream_t st);  // the same for n device control blocks
 // Light-prefix length of every row of g for delta (rows are sorted by weight).
 int count_light(const DevGraph &g, float delta, int32_t *nlight, cudaStream_t st);
 // Build (or rebuild for a new delta) the light rows of g; no-op when lr already holds delta.
