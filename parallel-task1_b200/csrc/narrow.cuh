@@ -15,33 +15,41 @@
 // and the one atomic that decides.
 //
 // Measured on a B200: a top-down step of the 1100 x 911 grid (662 rows on
-// average) 8.9 -> 3.7 us, an SSSP light round there 9.0 -> 6.8 us, BFS and SSSP
-// from one source 52 -> 38 ms; a BFS of six steps on 1,024 vertices 83 -> 62 us
-// with the call around it.  At RMAT scale 23 the step from a hub's neighbour
+// average) 8.9 -> 3.3 us, an SSSP light round there (342 rows) 9.0 -> 4.5 us, BFS
+// and SSSP from one source 47 -> 24 ms; a BFS of six steps on 1,024 vertices
+// 80 -> 57 us with the call around it.  At RMAT scale 23 the step from a hub's neighbour
 // (4,934 edges) takes 6 us instead of 72, because the chunk items of the hubs it
 // finds, which the bottom-up step after it does not read, are not written.
 //
 // A query starts here and goes on in the wide kernel (bfs_persistent /
 // sssp_persistent, which then also write the results back) as soon as a phase
-// has more edges than the cluster's shared memory holds next rows for; a query
-// that stays narrow ends here.
+// has too many edges, or more than a CTA's shared memory is sure to hold the
+// next rows for; a query that stays narrow ends here.
 //
-// Rows of the frontier are dealt round over the CTAs, 2^g lanes to a row and
+// Rows of the frontier stay with the CTA that found them, or are dealt round
+// when they are unevenly spread; 2^g lanes to a row and
 // four edges to a lane at a time, with g from the mean row length: the edges,
 // gathers and atomics of a lane are in flight together.
 #pragma once
 
-constexpr int kNarrowThreads = 1024;
+// One CTA an SM.  512 threads: with 768 or 1024 SSSP on that grid takes 22.3 or
+// 24.3 ms instead of 18.3 (the warps without a row still step through the
+// phase's bookkeeping).
+constexpr int kNarrowThreads = 512;
 constexpr int kNarrowCtas = 16;         // CTAs of the cluster (8 where the device cannot place 16)
-constexpr int kNarrowRows = 6144;       // rows a CTA's queue holds = edges a phase may have
+constexpr int kNarrowRows = 5120;       // rows a CTA's queue holds
+// Edges of the largest narrow phase.  The line is not sharp: with 16k, 64k or
+// 128k the grid, a uniform graph of 1M vertices and RMAT scale 16 measure the
+// same, since growing frontiers pass through this range in one step.
+constexpr unsigned kNarrowEdges = 32768;
 constexpr int kNarrowSeg = 128;         // longer rows are cut into segments of this many edges
 constexpr int kNarrowSegs = 512;        // segments after a row's first that a CTA's queue holds
-constexpr unsigned kNarrowFar = 4;      // far-pile entries per thread that a bucket opening may split (4096 a CTA)
+constexpr unsigned kNarrowFar = 4096;   // far-pile entries a CTA may split in a bucket opening
 constexpr int kNarrowOwn = 131072;      // graphs up to this size are also initialised and written back here
-enum NarrowCmd { kNarrowDone, kNarrowWide, kNarrowBudget, kNarrowPush, kNarrowPull, kNarrowHeavy, kNarrowOpen };
+enum NarrowCmd { kNarrowDone, kNarrowWide, kNarrowBudget, kNarrowPush, kNarrowPull, kNarrowHeavy, kNarrowOpen, kNarrowFlush };
 
 // What a CTA adds in one phase.
-struct NarrowCount {
+struct alignas(16) NarrowCount {
     unsigned rows;     // rows in its queue
     unsigned segs;     // further segments of long rows
     unsigned edges;    // and their edges
@@ -49,28 +57,32 @@ struct NarrowCount {
     unsigned scanned;  // edges expanded
     unsigned heavy;    // SSSP: entries added to its heavy list
     unsigned hedges;   // and their heavy edges
+    unsigned far;      // vertices for the far pile
     int far_key;       // SSSP: max of 0x7fffffff - distance bits pushed to the far pile
+    unsigned longest, hlongest;  // most edges of a row or segment, and of a heavy row
+    unsigned pad;
 };
+static_assert(sizeof(NarrowCount) == 48, "read as three 16-byte words");
 
 struct NarrowShared {
     // frontier rows of two phases, then the further segments
     int v[2][kNarrowRows + kNarrowSegs], begin[2][kNarrowRows + kNarrowSegs], len[2][kNarrowRows + kNarrowSegs];
     int heavy[2][kNarrowRows];               // SSSP heavy lists
+    int far[2][kNarrowRows];                 // vertices for the far pile, of two phases
     NarrowCount cnt[3];                      // ring over phases: being filled, being read, clear
-    // far piles' lengths (rank 0's are in use), a ring over bucket openings: the
-    // pile that grows, the one an opening fills, and one that is clear
-    unsigned nfar[3];
     unsigned first[kNarrowCtas + 1];         // rows and segments of the CTAs before each CTA
     unsigned mains[kNarrowCtas];             // rows among them
     // the phase, from the control warp
-    int cmd, g, in, ring, lists;
+    int cmd, g, in, ring, lists, dealt;
     unsigned rows, far_len, hbase;           // hbase: entries this CTA's heavy list holds already
     int level_next;
     float thr, told;
     unsigned round, h_start, f_start;
-    int hcur, fcur, opened;
+    int hcur, fcur;
+    unsigned far_n, far_at;                  // staged by this CTA in the phase before, and their place in the pile
+    int far_buf, far_pile;
     // log of the phase before (written out by an idle warp)
-    int log_phase, log_kind, log_dec, log_choice;
+    int log_phase, log_next, log_kind, log_dec, log_choice;  // log_phase -1: none; log_next: index of this phase
     unsigned log_size;
     unsigned long long log_scanned, log_state[5];
     float log_lo, log_hi;
@@ -132,7 +144,8 @@ __device__ __forceinline__ unsigned long long atom_min_if(unsigned long long *p,
 
 // Totals of a phase over the cluster (control warp; every lane gets them).
 struct NarrowTotal {
-    unsigned rows, units, edges, found, scanned, far_len;  // units: rows and segments
+    unsigned rows, units, edges, found, scanned;  // units: rows and segments
+    unsigned longest, most;                       // edges of the longest unit; units of the fullest CTA
     int far_key;
     NarrowCount rank;  // lane c: rank c's
 };
@@ -149,24 +162,30 @@ __device__ __forceinline__ unsigned scan_ranks(unsigned x)
 
 // Reads every CTA's counters of the phase that just ended.  (A CTA may be ahead
 // and add to what the next phase fills, so nothing that a phase adds to is read
-// while it runs, except the far pile's length, which is used only when no phase
-// adds to that pile.)
-__device__ __forceinline__ NarrowTotal narrow_totals(int ring, int opened)
+// while it runs.)
+__device__ __forceinline__ NarrowTotal narrow_totals(int ring)
 {
     NarrowShared &s = narrow();
     const unsigned lane = threadIdx.x & 31u, C = cluster_size();
     NarrowCount c{};
-    if (lane < C) c = on_rank(&s, lane)->cnt[ring];
+    if (lane < C) {
+        const uint4 *r = reinterpret_cast<const uint4 *>(&on_rank(&s, lane)->cnt[ring]);
+        uint4 *w = reinterpret_cast<uint4 *>(&c);
+        w[0] = r[0];
+        w[1] = r[1];
+        w[2] = r[2];
+    }
     c.segs = min(c.segs, (unsigned)kNarrowSegs);
     NarrowTotal t;
     t.rank = c;
-    t.far_len = *reinterpret_cast<volatile unsigned *>(&on_rank(&s, 0)->nfar[opened % 3]);
     t.rows = __reduce_add_sync(kFull, c.rows);
     t.units = __reduce_add_sync(kFull, c.rows + c.segs);
     t.edges = __reduce_add_sync(kFull, c.edges);
     t.found = __reduce_add_sync(kFull, c.found);
     t.scanned = __reduce_add_sync(kFull, c.scanned);
     t.far_key = __reduce_max_sync(kFull, c.far_key);
+    t.longest = __reduce_max_sync(kFull, c.longest);
+    t.most = __reduce_max_sync(kFull, c.rows + c.segs);
     return t;
 }
 
@@ -182,6 +201,24 @@ __device__ __forceinline__ void narrow_shares(unsigned rows, unsigned segs)
     }
 }
 
+// Whether a CTA's queues are sure to hold what a phase of `units` units of at
+// most `longest` edges adds to them, beside `held` entries: each edge adds at
+// most one row, one heavy entry or one far entry, and a CTA has at most its
+// share of the units (dealt round, or within narrow_deal's limit).
+__device__ __forceinline__ bool narrow_fits(unsigned units, unsigned edges, unsigned longest, unsigned held, unsigned C)
+{
+    const unsigned long long share = (unsigned long long)units / C + units / (4 * C) + 17u;
+    return min((unsigned long long)edges, share * longest) + held <= (unsigned long long)kNarrowRows;
+}
+
+// A phase's units stay with the CTAs that hold them while the fullest has not
+// much more than its share; otherwise they are dealt round (which reads them
+// across the cluster, some 1000 cycles).
+__device__ __forceinline__ bool narrow_deal(unsigned most, unsigned units, unsigned C)
+{
+    return most > units / C + units / (4 * C) + 16u;
+}
+
 // Lanes per row (as a power of two) for rows of edges / rows edges on average: four edges a lane.
 __device__ __forceinline__ int narrow_lanes(unsigned rows, unsigned edges)
 {
@@ -190,10 +227,14 @@ __device__ __forceinline__ int narrow_lanes(unsigned rows, unsigned edges)
     return g;
 }
 
-// Rank and index of row or segment r of the phase.
-__device__ __forceinline__ unsigned narrow_owner(unsigned r, unsigned &index)
+// Rank and index of row or segment r of the phase (dealt: of all, otherwise of this CTA's).
+__device__ __forceinline__ unsigned narrow_owner(unsigned r, unsigned &index, bool dealt, unsigned rank)
 {
     const NarrowShared &s = narrow();
+    if (!dealt) {
+        index = r < s.mains[rank] ? r : r + (kNarrowRows - s.mains[rank]);
+        return rank;
+    }
     unsigned c = 0;
 #pragma unroll
     for (unsigned d = kNarrowCtas / 2; d; d >>= 1)
@@ -203,10 +244,10 @@ __device__ __forceinline__ unsigned narrow_owner(unsigned r, unsigned &index)
     return c;
 }
 
-__device__ __forceinline__ void narrow_push_row(int out, NarrowCount &c, int v, int begin, int len)
+// Row i of queue `out`; `longest` is raised to its edges (or its segments').
+__device__ __forceinline__ void narrow_put_row(int out, NarrowCount &c, unsigned i, int v, int begin, int len, unsigned &longest)
 {
     NarrowShared &s = narrow();
-    const unsigned i = atomicAdd(&c.rows, 1u);
     if (len > kNarrowSeg && len <= kNarrowRows) {
         // A long row in few lanes would be a long chain: its segments are units
         // of their own.  Where they do not fit, the row stays whole: the first
@@ -232,6 +273,7 @@ __device__ __forceinline__ void narrow_push_row(int out, NarrowCount &c, int v, 
             }
         }
     }
+    longest = max(longest, (unsigned)len);
     s.v[out][i] = v;
     s.begin[out][i] = begin;
     s.len[out][i] = len;
@@ -256,7 +298,7 @@ __device__ __noinline__ void narrow_write_log(Ctl *ctl)
 #pragma unroll
         for (int k = 0; k < 5; k++) x[k] = s.log_state[k];
         ctl->dec_choice[i] = (unsigned char)s.log_choice;
-        ctl->dec_phase[i] = s.log_phase + 1;
+        ctl->dec_phase[i] = s.log_next;
         ctl->dec_lo[i] = s.log_lo;
         ctl->dec_hi[i] = s.log_hi;
     }
@@ -335,16 +377,14 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
     const bool own = a.V <= kNarrowOwn;
     if (own) bfs_init(a, rank * kNarrowThreads + tid, nth);
     if (tid == 0) {
-        for (int k = 0; k < 3; k++) {
-            s.cnt[k] = NarrowCount{};
-            s.nfar[k] = 0;
-        }
+        for (int k = 0; k < 3; k++) s.cnt[k] = NarrowCount{};
         if (rank == 0) {
             const int b = __ldg(&a.out_off[src]), d = __ldg(&a.out_off[src + 1]) - b;
             s.cnt[0].found = 1;
             s.cnt[0].edges = (unsigned)d;
             if (d > 0) {
-                narrow_push_row(0, s.cnt[0], src, b, d);
+                s.cnt[0].rows = 1;
+                narrow_put_row(0, s.cnt[0], 0, src, b, d, s.cnt[0].longest);
             }
         }
     }
@@ -355,7 +395,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
     int L = 0, dir = 0, bu = 0;
     for (int p = 0;; p++) {
         if (tid < 32) {
-            const NarrowTotal t = narrow_totals(p % 3, 0);
+            const NarrowTotal t = narrow_totals(p % 3);
             narrow_shares(t.rank.rows, t.rank.segs);
             const unsigned long long done_nf = nf;
             if (p > 0) {
@@ -367,25 +407,30 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
             scanned += t.scanned;
             int plain = dir;
             if (dir == 0) {
-                if ((double)t.edges > (double)mu / a.alpha) plain = 1;
-            } else if (!(nf >= nf_prev || (double)nf > (double)a.V / a.beta)) {
+                if ((double)t.edges * a.alpha > (double)mu) plain = 1;
+            } else if (!(nf >= nf_prev || (double)nf * a.beta > (double)a.V)) {
                 plain = 0;
             }
             const int d = a.force_dir >= 0 ? (L == 0 ? 0 : a.force_dir) : plain;
             int cmd = d ? kNarrowPull : kNarrowPush;
             if (nf == 0) cmd = kNarrowDone;
             else if (L >= a.max_steps) cmd = kNarrowBudget;
-            else if (!alone && (d || t.edges > (unsigned)kNarrowRows)) cmd = kNarrowWide;
+            else if (!alone && (d || t.edges > kNarrowEdges || !narrow_fits(t.units, t.edges, t.longest, 0, C))) cmd = kNarrowWide;
             const bool step = cmd == kNarrowPush || cmd == kNarrowPull;
             if (tid == 0) {
                 s.cmd = cmd;
                 s.rows = t.units;
                 s.g = narrow_lanes(t.units, t.edges);
+                s.dealt = narrow_deal(t.most, t.units, C);
                 s.in = p & 1;
                 s.ring = (p + 1) % 3;
                 s.level_next = L + 1;
                 s.lists = cmd == kNarrowWide && !d;  // a bottom-up step needs none
+                s.cnt[(p + 2) % 3] = NarrowCount{};
+            }
+            if (tid == 0 && rank == C - 1) {  // for the log
                 s.log_phase = p - 1;
+                s.log_next = p;
                 s.log_kind = dir;
                 s.log_size = (unsigned)done_nf;
                 s.log_scanned = scanned;
@@ -397,12 +442,13 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
                 s.log_state[2] = mu;
                 s.log_state[3] = nf_prev;
                 s.log_state[4] = (unsigned long long)(unsigned)L | (unsigned long long)dir << 32 | (unsigned long long)plain << 33;
-                s.cnt[(p + 2) % 3] = NarrowCount{};
-                if (rank == C - 1 && step && L < kMaxTrace) {
+                if (step && L < kMaxTrace) {
                     ctl->dirs[L] = (unsigned char)d;
                     ctl->frontier[L] = (unsigned)nf;
                 }
-                if (rank == 0 && !step) {
+            }
+            if (tid == 0 && rank == 0) {
+                if (!step) {
                     ctl->steps = L;
                     ctl->bottom_up_steps = bu;
                     ctl->buckets = 0;
@@ -430,13 +476,16 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
         if (narrow_logger()) narrow_write_log(ctl);
         const int cmd = s.cmd, in = s.in, out = in ^ 1;
         NarrowCount &c = s.cnt[s.ring];
-        unsigned edges = 0, found = 0, expanded = 0;
+        unsigned edges = 0, found = 0, expanded = 0, longest = 0;
         if (cmd == kNarrowPush) {
-            const unsigned rows = s.rows;
+            const bool dealt = s.dealt;
+            const unsigned rows = dealt ? s.rows : s.first[rank + 1] - s.first[rank];
             const int g = s.g, sub = (int)(tid & ((1u << g) - 1u));
-            for (unsigned r = (tid >> g) * C + rank; r < rows; r += (kNarrowThreads >> g) * C) {
+            const unsigned r0 = dealt ? (tid >> g) * C + rank : tid >> g, step = (kNarrowThreads >> g) * (dealt ? C : 1u);
+            for (unsigned r = r0; r < rows; r += step) {
                 unsigned i;
-                const NarrowShared *o = on_rank(&s, narrow_owner(r, i));
+                const unsigned owner = narrow_owner(r, i, dealt, rank);
+                const NarrowShared *o = dealt ? on_rank(&s, owner) : &s;
                 const int len = o->len[in][i], b = o->begin[in][i], end = b + len;
                 if (sub == 0) expanded += (unsigned)len;
                 for (int e = b + 4 * sub; e < end; e += 4 << g) {
@@ -453,13 +502,23 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
                         o0[j] = ok ? __ldg(&a.out_off[v[j]]) : 0;
                         o1[j] = ok ? __ldg(&a.out_off[v[j] + 1]) : 0;
                     }
+                    unsigned rows_new = 0;
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        if (e + j >= end || (old[j] >> (v[j] & 31) & 1u)) continue;
-                        reinterpret_cast<int *>(a.value)[v[j]] = s.level_next;
-                        found++;
-                        edges += (unsigned)(o1[j] - o0[j]);
-                        if (o1[j] > o0[j]) narrow_push_row(out, c, v[j], o0[j], o1[j] - o0[j]);
+                        const bool fresh = e + j < end && !(old[j] >> (v[j] & 31) & 1u);
+                        if (fresh) reinterpret_cast<int *>(a.value)[v[j]] = s.level_next;
+                        found += fresh;
+                        if (!fresh) o1[j] = o0[j];
+                        rows_new += o1[j] > o0[j];
+                    }
+                    if (rows_new) {
+                        unsigned at = atomicAdd(&c.rows, rows_new);
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            if (o1[j] <= o0[j]) continue;
+                            edges += (unsigned)(o1[j] - o0[j]);
+                            narrow_put_row(out, c, at++, v[j], o0[j], o1[j] - o0[j], longest);
+                        }
                     }
                 }
             }
@@ -484,7 +543,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
                 const int o0 = __ldg(&a.out_off[v]), o1 = __ldg(&a.out_off[v + 1]);
                 found++;
                 edges += (unsigned)(o1 - o0);
-                if (o1 > o0) narrow_push_row(out, c, (int)v, o0, o1 - o0);
+                if (o1 > o0) narrow_put_row(out, c, atomicAdd(&c.rows, 1u), (int)v, o0, o1 - o0, longest);
             }
         } else {
             break;
@@ -494,10 +553,12 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
             edges = __reduce_add_sync(kFull, edges);
             found = __reduce_add_sync(kFull, found);
             expanded = __reduce_add_sync(kFull, expanded);
+            longest = __reduce_max_sync(kFull, longest);
             if ((tid & 31u) == 0) {
                 atomicAdd(&c.edges, edges);
                 atomicAdd(&c.found, found);
                 atomicAdd(&c.scanned, expanded);
+                atomicMax(&c.longest, longest);
             }
         }
         cluster_sync();
@@ -513,8 +574,8 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
         }
     }
     cluster_sync();  // the logs are written
-    const int n = min((int)__ldcg(&ctl->ndec), kMaxDec);
-    for (int i = (int)gtid; i < n; i += (int)nth) {
+    const int decisions = min((int)__ldcg(&ctl->ndec), kMaxDec);
+    for (int i = (int)gtid; i < decisions; i += (int)nth) {
         unsigned long long x[5];
 #pragma unroll
         for (int k = 0; k < 5; k++) x[k] = __ldcg(reinterpret_cast<unsigned long long *>(ctl->dec_x[i]) + k);
@@ -541,30 +602,44 @@ __global__ void __launch_bounds__(256) sssp_init_kernel(TravArgs a)
     sssp_init(a, blockIdx.x * 256 + threadIdx.x, gridDim.x * 256);
 }
 
-// The next index from a counter on another CTA: one remote atomic for the
-// lanes that are here together.
-__device__ __forceinline__ unsigned narrow_take(unsigned *n)
-{
-    const unsigned m = __activemask(), leader = (unsigned)__ffs(m) - 1u;
-    unsigned base = 0;
-    if ((threadIdx.x & 31u) == leader) base = atomicAdd(n, (unsigned)__popc(m));
-    return __shfl_sync(m, base, (int)leader) + __popc(m & lanemask_lt());
-}
+// Per-thread sums of a phase.
+struct NarrowSums {
+    unsigned edges, hedges, expanded, longest, hlongest;
+    int far_key;
+};
 
-// Vertex v was lowered below the bound (or opened): its light row joins the
-// next frontier, its heavy row the heavy list.
-__device__ __forceinline__ void narrow_add(const TravArgs &a, NarrowCount &c, int out, int hcur, int v, bool light, bool heavy,
-                                           int lb, int le, int hedges, unsigned &edges, unsigned &hsum,
-                                           unsigned hbase)
+// What a thread adds for its N vertices v[j] at once, one reservation a list:
+// bit 0 of push[j]: its light row [lb, le) joins the next frontier; bit 1: its
+// heavy row (hlen edges) the heavy list hcur; bit 2: it joins the far pile.
+template <int N>
+__device__ __forceinline__ void narrow_add(NarrowCount &c, int out, int hcur, unsigned hbase, const int (&v)[N],
+                                           const unsigned (&push)[N], const int (&lb)[N], const int (&le)[N],
+                                           const int (&hlen)[N], NarrowSums &n)
 {
     NarrowShared &s = narrow();
-    if (light) {
-        edges += (unsigned)(le - lb);
-        narrow_push_row(out, c, v, lb, le - lb);
+    unsigned nl = 0, nh = 0, nf = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        nl += push[j] & 1u;
+        nh += push[j] >> 1 & 1u;
+        nf += push[j] >> 2;
     }
-    if (heavy) {
-        hsum += (unsigned)hedges;
-        s.heavy[hcur][hbase + atomicAdd(&c.heavy, 1u)] = v;
+    unsigned al = 0, ah = 0, af = 0;
+    if (nl) al = atomicAdd(&c.rows, nl);
+    if (nh) ah = hbase + atomicAdd(&c.heavy, nh);
+    if (nf) af = atomicAdd(&c.far, nf);
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        if (push[j] & 1u) {
+            n.edges += (unsigned)(le[j] - lb[j]);
+            narrow_put_row(out, c, al++, v[j], lb[j], le[j] - lb[j], n.longest);
+        }
+        if (push[j] & 2u) {
+            n.hedges += (unsigned)hlen[j];
+            n.hlongest = max(n.hlongest, (unsigned)hlen[j]);
+            s.heavy[hcur][ah++] = v[j];
+        }
+        if (push[j] & 4u) s.far[out][af++] = v[j];
     }
 }
 
@@ -581,20 +656,18 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
     if (a.mlp)
         for (unsigned i = tid; i < (unsigned)mlp_param_count(kSsspOut); i += kNarrowThreads) s.mlp[i] = __ldg(&a.mlp[i]);
     if (tid == 0) {
-        for (int k = 0; k < 3; k++) {
-            s.cnt[k] = NarrowCount{};
-            s.nfar[k] = 0;
-        }
+        for (int k = 0; k < 3; k++) s.cnt[k] = NarrowCount{};
         if (rank == 0) {
             const int b = __ldg(&lo_off[src]), d = __ldg(&lo_off[src + 1]) - b;
             const int deg = __ldg(&a.out_off[src + 1]) - __ldg(&a.out_off[src]);
             s.cnt[0].edges = (unsigned)d;
             if (d > 0) {
-                narrow_push_row(0, s.cnt[0], src, b, d);
+                s.cnt[0].rows = 1;
+                narrow_put_row(0, s.cnt[0], 0, src, b, d, s.cnt[0].longest);
             }
             if (deg > d) {
                 s.cnt[0].heavy = 1;
-                s.cnt[0].hedges = (unsigned)(deg - d);
+                s.cnt[0].hedges = s.cnt[0].hlongest = (unsigned)(deg - d);
                 s.heavy[0][0] = src;
             }
         }
@@ -603,54 +676,64 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
     if (rank == 0 && tid == 0) ctl->t0_ns = globaltimer();
     // state of the control warp
     float thr = a.delta > 0.0f ? a.delta : INFINITY, lo = 0.0f;
-    unsigned nheavy = 0, hedges = 0;  // lane c: entries and edges of rank c's heavy list
-    int hcur = 0, fcur = 0, opened = 0, steps = 0, buckets = 1, last = -1, min_far = (int)kFltMaxBits;
+    unsigned nheavy = 0, hedges = 0, hlongest = 0;  // lane c: entries, edges and longest row of rank c's heavy list
+    unsigned far_len = 0;             // far pile in memory
+    int hcur = 0, fcur = 0, steps = 0, buckets = 1, last = -1, flushes = 0, min_far = (int)kFltMaxBits;
     unsigned round = 1, h_start = 1, f_start = 1, last_size = 0;
     unsigned long long scanned = 0;
     for (int p = 0;; p++) {
         if (tid < 32) {
-            const NarrowTotal t = narrow_totals(p % 3, opened);
+            const NarrowTotal t = narrow_totals(p % 3);
             nheavy += t.rank.heavy;
             hedges += t.rank.hedges;
+            hlongest = max(hlongest, t.rank.hlongest);
             const unsigned heavy = __reduce_add_sync(kFull, nheavy), heavy_edges = __reduce_add_sync(kFull, hedges);
-            const unsigned max_heavy = __reduce_max_sync(kFull, nheavy);
+            const unsigned max_heavy = __reduce_max_sync(kFull, nheavy), heavy_longest = __reduce_max_sync(kFull, hlongest);
             scanned += t.scanned;
             const int far_bits = t.far_key > 0 ? 0x7fffffff - t.far_key : (int)kFltMaxBits;
             min_far = last == 4 ? far_bits : min(min_far, far_bits);
+            // what the last phase staged for the far pile joins it after what is there
+            const unsigned staged_incl = scan_ranks(t.rank.far);
+            const unsigned staged = __shfl_sync(kFull, staged_incl, 31), most_staged = __reduce_max_sync(kFull, t.rank.far);
+            const unsigned far_n = __shfl_sync(kFull, t.rank.far, (int)rank);
+            const unsigned far_at = far_len + __shfl_sync(kFull, staged_incl, (int)rank) - far_n;
             // the next phase
             int cmd;
             unsigned size = 0;
             if (t.rows > 0) {
                 cmd = kNarrowPush;
                 size = t.rows;
-                if (!alone && (t.edges > (unsigned)kNarrowRows || max_heavy + t.edges > (unsigned)kNarrowRows)) cmd = kNarrowWide;
+                if (!alone && (t.edges > kNarrowEdges || !narrow_fits(t.units, t.edges, t.longest, max_heavy, C))) cmd = kNarrowWide;
             } else if (heavy > 0) {
                 cmd = kNarrowHeavy;
                 size = heavy;
-                if (!alone && heavy_edges > (unsigned)kNarrowRows) cmd = kNarrowWide;
-            } else if (t.far_len > 0) {
+                if (!alone && (heavy_edges > kNarrowEdges || !narrow_fits(heavy, heavy_edges, heavy_longest, 0, C))) cmd = kNarrowWide;
+            } else if (far_len + staged > 0) {
+                // every entry may join a CTA's queue or its next staging; where a
+                // CTA would get too many, they are written out first
                 cmd = kNarrowOpen;
-                size = t.far_len;
-                if (!alone && t.far_len > kNarrowFar * nth) cmd = kNarrowWide;
+                size = far_len + staged;
+                if (!alone && far_len + staged > kNarrowFar * C) cmd = kNarrowWide;
+                else if (staged > 0 && far_len / C + kNarrowThreads + most_staged > (unsigned)kNarrowRows) cmd = kNarrowFlush;
             } else {
                 cmd = kNarrowDone;
             }
             if (cmd != kNarrowDone && steps + buckets >= a.max_steps) cmd = kNarrowBudget;
             narrow_shares(cmd == kNarrowHeavy ? nheavy : t.rank.rows, cmd == kNarrowHeavy ? 0u : t.rank.segs);
             const unsigned mine = __shfl_sync(kFull, nheavy, (int)rank);
-            if (cmd == kNarrowHeavy) nheavy = hedges = 0;  // the list is used up; the other one starts empty
+            if (cmd == kNarrowHeavy) nheavy = hedges = hlongest = 0;  // the list is used up; the other one starts empty
             int option = -1;
             float told = thr;
             unsigned long long st0 = 0, st1 = 0, st2 = 0;
             if (cmd == kNarrowOpen) {
                 // bound = max(old, min far) + width, as in sssp_query
                 option = 0;
-                st0 = (unsigned long long)t.far_len | (unsigned long long)(unsigned)steps << 32;
+                st0 = (unsigned long long)size | (unsigned long long)(unsigned)steps << 32;
                 st1 = (unsigned long long)(unsigned)buckets;
                 st2 = (unsigned long long)(unsigned)min_far | (unsigned long long)__float_as_uint(thr) << 32;
                 if (a.mlp)
                     option = mlp_argmax_warp<kSsspOut>(s.mlp,
-                                                       sssp_features(steps, t.far_len, __int_as_float(min_far), thr, a.delta, a.V,
+                                                       sssp_features(steps, size, __int_as_float(min_far), thr, a.delta, a.V,
                                                                      a.E, buckets, a.mean_w, a.max_deg),
                                                        0, a.mlp_margin);
                 const float width = a.delta * sssp_width_scale(option);
@@ -661,12 +744,17 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                 h_start = f_start = round;
             }
             if (cmd == kNarrowHeavy) h_start = round;
-            const bool more = cmd == kNarrowPush || cmd == kNarrowHeavy || cmd == kNarrowOpen;
+            const bool more = cmd >= kNarrowPush;
             if (tid == 0) {
                 s.cmd = cmd;
                 s.rows = cmd == kNarrowPush ? t.units : size;
-                s.far_len = t.far_len;
+                s.far_len = far_len;
+                s.far_n = far_n;
+                s.far_at = far_at;
+                s.far_buf = p & 1;
+                s.far_pile = fcur;
                 s.hbase = cmd == kNarrowHeavy ? 0u : mine;
+                s.dealt = cmd == kNarrowHeavy ? narrow_deal(max_heavy, heavy, C) : narrow_deal(t.most, t.units, C);
                 s.g = cmd == kNarrowHeavy ? narrow_lanes(heavy, heavy_edges) : narrow_lanes(t.units, t.edges);
                 s.in = p & 1;
                 s.ring = (p + 1) % 3;
@@ -677,8 +765,11 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                 s.f_start = f_start;
                 s.hcur = hcur;
                 s.fcur = fcur;
-                s.opened = opened;
-                s.log_phase = p - 1;
+                s.cnt[(p + 2) % 3] = NarrowCount{};
+            }
+            if (tid == 0 && rank == C - 1) {  // for the log
+                s.log_phase = last >= 0 ? p - 1 - flushes : -1;
+                s.log_next = p - flushes;
                 s.log_kind = last;
                 s.log_size = last_size;
                 s.log_scanned = scanned;
@@ -690,14 +781,14 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                 s.log_state[1] = st1;
                 s.log_state[2] = st2;
                 s.log_state[3] = s.log_state[4] = 0;
-                s.cnt[(p + 2) % 3] = NarrowCount{};
-                if (cmd == kNarrowOpen) s.nfar[(opened + 2) % 3] = 0;
-                if (cmd == kNarrowPush && rank == C - 1 && steps < kMaxTrace) ctl->frontier[steps] = size;
-                if (rank == 0 && !more) {
+                if (cmd == kNarrowPush && steps < kMaxTrace) ctl->frontier[steps] = size;
+            }
+            if (tid == 0 && rank == 0) {
+                if (!more) {
                     ctl->steps = steps;
                     ctl->buckets = buckets;
                     ctl->bottom_up_steps = 0;
-                    ctl->nphase = p;
+                    ctl->nphase = p - flushes;
                     ctl->ndec = buckets - 1;
                     ctl->edges_scanned = scanned;
                     if (cmd == kNarrowBudget) ctl->err = kErrBudget;
@@ -707,7 +798,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                     r.steps = steps;
                     r.buckets = buckets;
                     r.scanned = scanned;
-                    r.far_len = t.far_len;
+                    r.far_len = far_len + staged;
                     r.fcur = fcur;
                     r.min_far = min_far;
                     r.thr = thr;
@@ -717,14 +808,19 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                     r.f_start = f_start;
                 }
             }
-            last = cmd == kNarrowPush ? 3 : cmd == kNarrowHeavy ? 5 : 4;
-            last_size = size;
+            far_len = cmd == kNarrowOpen ? 0 : far_len + staged;
+            if (cmd == kNarrowFlush) {
+                last = -1;  // no phase of the query: nothing to count or log
+                flushes++;
+            } else {
+                last = cmd == kNarrowPush ? 3 : cmd == kNarrowHeavy ? 5 : 4;
+                last_size = size;
+            }
             round++;
             if (cmd == kNarrowOpen) {
                 fcur ^= 1;
-                opened++;
                 buckets++;
-            } else {
+            } else if (cmd != kNarrowFlush) {
                 steps++;
                 if (cmd == kNarrowHeavy) hcur ^= 1;
             }
@@ -733,20 +829,24 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
         if (narrow_logger()) narrow_write_log(ctl);
         const int cmd = s.cmd, in = s.in, out = in ^ 1;
         NarrowCount &c = s.cnt[s.ring];
-        unsigned edges = 0, hsum = 0, expanded = 0;
-        int far_key = 0;
+        NarrowSums n{0, 0, 0, 0, 0, 0};
+        if (cmd != kNarrowOpen) {
+            int32_t *pile = s.far_pile ? a.far1 : a.far0;
+            for (unsigned i = tid; i < s.far_n; i += kNarrowThreads) pile[s.far_at + i] = s.far[s.far_buf][i];
+        }
         if (cmd == kNarrowPush || cmd == kNarrowHeavy) {
             const bool heavy_rows = cmd == kNarrowHeavy, packed = !heavy_rows && a.nlight;
             const int hc = heavy_rows ? s.hcur ^ 1 : s.hcur;  // the heavy list that grows
-            const unsigned rows = s.rows, round_ = s.round;
+            const bool dealt = s.dealt;
+            const unsigned rows = dealt ? s.rows : s.first[rank + 1] - s.first[rank], round_ = s.round;
             const int g = s.g, sub = (int)(tid & ((1u << g) - 1u));
+            const unsigned r0 = dealt ? (tid >> g) * C + rank : tid >> g, step = (kNarrowThreads >> g) * (dealt ? C : 1u);
             const float bound = s.thr;
             const unsigned hbase = s.hbase;
-            unsigned *nfar = &on_rank(&s, 0)->nfar[s.opened % 3];
-            int32_t *far = s.fcur ? a.far1 : a.far0;
-            for (unsigned r = (tid >> g) * C + rank; r < rows; r += (kNarrowThreads >> g) * C) {
+            for (unsigned r = r0; r < rows; r += step) {
                 unsigned i;
-                const NarrowShared *o = on_rank(&s, narrow_owner(r, i));
+                const unsigned owner = narrow_owner(r, i, dealt, rank);
+                const NarrowShared *o = dealt ? on_rank(&s, owner) : &s;
                 int u, b, end;
                 if (heavy_rows) {
                     u = o->heavy[s.hcur][i];
@@ -757,7 +857,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                     b = o->begin[in][i];
                     end = b + o->len[in][i];
                 }
-                if (sub == 0) expanded += (unsigned)(end - b);
+                if (sub == 0) n.expanded += (unsigned)(end - b);
                 const float du = dist_of(__ldcg(&a.dist[u]));
                 for (int e = b + 4 * sub; e < end; e += 4 << g) {
                     int v[4];
@@ -790,60 +890,73 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                         o0[j] = ok[j] ? __ldg(&a.out_off[v[j]]) : 0;
                         o1[j] = ok[j] ? __ldg(&a.out_off[v[j] + 1]) : 0;
                     }
+                    unsigned push[4];
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
-                        const float od = dist_of(old[j]);
-                        if (!ok[j] || !(nd[j] < od)) continue;
                         // push decisions as in SsspVisit::drain
+                        const float od = dist_of(old[j]);
                         const unsigned cls = (unsigned)old[j] & kClsMask, orr = (unsigned)old[j] >> kClsBits;
-                        if (nd[j] < bound) {
-                            const bool below = od < bound;
-                            narrow_add(a, c, out, hc, v[j], (cls & kClsLight) && !(below && orr >= round_),
-                                       (cls & kClsHeavy) && !(below && orr >= s.h_start), l0[j], l1[j],
-                                       (o1[j] - o0[j]) - (l1[j] - l0[j]), edges, hsum, hbase);
-                        } else if (!(orr >= s.f_start)) {
-                            far[narrow_take(nfar)] = v[j];
-                            far_key = max(far_key, 0x7fffffff - __float_as_int(nd[j]));
+                        push[j] = 0;
+                        if (ok[j] && nd[j] < od) {
+                            if (nd[j] < bound) {
+                                const bool below = od < bound;
+                                push[j] = ((cls & kClsLight) && !(below && orr >= round_) ? 1u : 0u) |
+                                          ((cls & kClsHeavy) && !(below && orr >= s.h_start) ? 2u : 0u);
+                            } else if (!(orr >= s.f_start)) {
+                                push[j] = 4u;
+                                n.far_key = max(n.far_key, 0x7fffffff - __float_as_int(nd[j]));
+                            }
                         }
+                        o0[j] = (o1[j] - o0[j]) - (l1[j] - l0[j]);  // heavy edges
                     }
+                    narrow_add(c, out, hc, hbase, v, push, l0, l1, o0, n);
                 }
             }
         } else if (cmd == kNarrowOpen) {
+            // the pile in memory, shared out over the cluster, and what this CTA
+            // staged in the phase before
             const int32_t *fp = s.fcur ? a.far1 : a.far0;
-            int32_t *far = s.fcur ? a.far0 : a.far1;
-            unsigned *nfar = &on_rank(&s, 0)->nfar[(s.opened + 1) % 3];
-            for (unsigned i = gtid; i < s.far_len; i += nth) {
-                const int v = __ldcg(&fp[i]);
+            const unsigned share = s.far_len > gtid ? (s.far_len - gtid + nth - 1) / nth : 0u;
+            const unsigned staged = s.far_n > tid ? (s.far_n - tid + kNarrowThreads - 1) / kNarrowThreads : 0u;
+            for (unsigned k = 0; k < share + staged; k++) {
+                const int v = k < share ? __ldcg(&fp[gtid + k * nth]) : s.far[s.far_buf][tid + (k - share) * kNarrowThreads];
                 const unsigned long long dv = __ldcg(&a.dist[v]);
                 const unsigned cls = (unsigned)dv & kClsMask;
                 const float d = dist_of(dv);
                 if (!(d >= s.told)) continue;
                 // stamp the word with this round, keeping the distance
                 atomicMax(&a.dist[v], pack_dist(d, s.round << kClsBits | cls));
-                if (d < s.thr) {
-                    const int l0 = __ldg(&lo_off[v]), l1 = __ldg(&lo_off[v + 1]);
-                    const int deg = __ldg(&a.out_off[v + 1]) - __ldg(&a.out_off[v]);
-                    narrow_add(a, c, out, s.hcur, v, cls & kClsLight, cls & kClsHeavy, l0, l1, deg - (l1 - l0), edges, hsum,
-                               s.hbase);
+                const bool in_bucket = d < s.thr;
+                const int vs[1] = {v};
+                int l0[1] = {0}, l1[1] = {0}, hl[1] = {0};
+                const unsigned push[1] = {in_bucket ? (cls & kClsLight ? 1u : 0u) | (cls & kClsHeavy ? 2u : 0u) : 4u};
+                if (in_bucket) {
+                    l0[0] = __ldg(&lo_off[v]);
+                    l1[0] = __ldg(&lo_off[v + 1]);
+                    hl[0] = __ldg(&a.out_off[v + 1]) - __ldg(&a.out_off[v]) - (l1[0] - l0[0]);
                 } else {
-                    far[narrow_take(nfar)] = v;
-                    far_key = max(far_key, 0x7fffffff - __float_as_int(d));
+                    n.far_key = max(n.far_key, 0x7fffffff - __float_as_int(d));
                 }
+                narrow_add(c, out, s.hcur, s.hbase, vs, push, l0, l1, hl, n);
             }
-        } else {
+        } else if (cmd != kNarrowFlush) {
             break;
         }
         __syncwarp();
-        if (__any_sync(kFull, (edges | hsum | expanded | (unsigned)far_key) != 0u)) {
-            edges = __reduce_add_sync(kFull, edges);
-            hsum = __reduce_add_sync(kFull, hsum);
-            expanded = __reduce_add_sync(kFull, expanded);
-            far_key = __reduce_max_sync(kFull, far_key);
+        if (__any_sync(kFull, (n.edges | n.hedges | n.expanded | (unsigned)n.far_key) != 0u)) {
+            n.edges = __reduce_add_sync(kFull, n.edges);
+            n.hedges = __reduce_add_sync(kFull, n.hedges);
+            n.expanded = __reduce_add_sync(kFull, n.expanded);
+            n.far_key = __reduce_max_sync(kFull, n.far_key);
+            n.longest = __reduce_max_sync(kFull, n.longest);
+            n.hlongest = __reduce_max_sync(kFull, n.hlongest);
             if (lane == 0) {
-                atomicAdd(&c.edges, edges);
-                atomicAdd(&c.hedges, hsum);
-                atomicAdd(&c.scanned, expanded);
-                atomicMax(&c.far_key, far_key);
+                atomicAdd(&c.edges, n.edges);
+                atomicAdd(&c.hedges, n.hedges);
+                atomicAdd(&c.scanned, n.expanded);
+                atomicMax(&c.far_key, n.far_key);
+                atomicMax(&c.longest, n.longest);
+                atomicMax(&c.hlongest, n.hlongest);
             }
         }
         cluster_sync();
@@ -867,8 +980,8 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
         }
     }
     cluster_sync();  // the logs are written
-    const int n = min((int)__ldcg(&ctl->ndec), kMaxDec);
-    for (int i = (int)gtid; i < n; i += (int)nth) {
+    const int decisions = min((int)__ldcg(&ctl->ndec), kMaxDec);
+    for (int i = (int)gtid; i < decisions; i += (int)nth) {
         unsigned long long x[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) x[k] = __ldcg(reinterpret_cast<unsigned long long *>(ctl->dec_x[i]) + k);

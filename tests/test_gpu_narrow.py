@@ -40,12 +40,12 @@ def _grid(h, wd, seed):
     return h * wd, s, d, np.random.default_rng(seed).integers(1, 100, len(s)).astype(np.float32)
 
 
-@pytest.mark.parametrize("h,wd", [(1, 3), (64, 96), (64, 97), (5, 3000), (362, 362), (400, 331)])
+@pytest.mark.parametrize("h,wd", [(1, 3), (64, 80), (64, 81), (64, 96), (64, 97), (5, 3000), (362, 362), (400, 331)])
 def test_grids_stay_narrow(h, wd):
     _check(*_grid(h, wd, h), src=h * wd // 2)
 
 
-@pytest.mark.parametrize("deg", [0, 1, 127, 128, 129, 640, 6143, 6144, 6145, 20_000])
+@pytest.mark.parametrize("deg", [0, 1, 127, 128, 129, 640, 5119, 5120, 5121, 6143, 6144, 6145, 20_000])
 def test_rows_at_the_segment_and_queue_limits(deg):
     """A hub behind a path, with `deg` out-edges to leaves that join again and go on."""
     V = deg + 8
@@ -55,7 +55,7 @@ def test_rows_at_the_segment_and_queue_limits(deg):
     _check(V, s, d, (rng.integers(0, 9, len(s)) / 8).astype(np.float32), 0)
 
 
-@pytest.mark.parametrize("V,E,seed", [(6144, 30_000, 1), (6145, 30_000, 2), (6144, 300_000, 3), (131_072, 400_000, 4),
+@pytest.mark.parametrize("V,E,seed", [(5120, 30_000, 8), (5121, 30_000, 9), (6144, 30_000, 1), (6145, 30_000, 2), (6144, 300_000, 3), (131_072, 400_000, 4),
                                       (131_073, 400_000, 5), (3000, 262_144, 6), (40_000, 60_000, 7)])
 def test_random_graphs_change_over(V, E, seed):
     rng = np.random.default_rng(seed)
@@ -104,3 +104,16 @@ def test_long_rows_beyond_the_segments_of_a_queue(first, fan):
     d = np.concatenate([np.arange(1, first + 1), rng.integers(0, V, first * fan)])
     assert len(s) <= 1 << 18
     _check(V, s, d, rng.uniform(0.01, 1.0, len(s)), 0, deltas=(0.0, 0.3))
+
+
+@pytest.mark.parametrize("width", [1, 15, 16, 17, 500, 2500, 9000])
+def test_frontiers_of_one_width(width):
+    """Ladders: `width` paths side by side with a common root, so that every phase has as many rows; with cross edges
+    that make the rows of one path longer than the others' (rows stay with their block, or are dealt round)."""
+    n = 12
+    idx = 1 + np.arange(n * width).reshape(n, width)
+    s = [np.zeros(width), idx[:-1].ravel(), np.repeat(idx[:-1, 0], min(width, 400))]
+    d = [idx[0], idx[1:].ravel(), np.concatenate([row[: min(width, 400)] for row in idx[1:]])]
+    s, d = np.concatenate(s).astype(np.int64), np.concatenate(d)
+    rng = np.random.default_rng(width)
+    _check(1 + n * width, s, d, (rng.integers(1, 20, len(s)) / 4).astype(np.float32), 0, deltas=(0.0, 1.0, 3.0))
