@@ -202,6 +202,7 @@ struct TravArgs {
     int32_t color_want;
     // SSSP options
     float delta;           // +inf = Bellman-Ford
+    int32_t near_rows;     // gathered distances of vertices below this may come from L1 (see gather_near)
     float mean_w;          // mean edge weight of the graph
     int32_t max_deg;       // largest out-degree of the graph
     // output (original ids); nullptr = leave results in `value`

@@ -117,6 +117,49 @@ __device__ __forceinline__ unsigned long long ld_gather(const unsigned long long
 #endif
 }
 
+// Gathers of distances that a relaxation is only tested against, of vertices below
+// near_rows from L1 where they are there.  Vertices are numbered by falling
+// degree, so the 16 distances of a 128-byte line near the start are those of 16
+// hubs, and on an RMAT graph one line takes 1.6% of all gathers: ncu showed the
+// L2 slice it lives in at 69% of its tag rate over a whole Bellman-Ford query
+// (scale 21), the slices' mean at 24%, and nothing else above 30%.  A distance in
+// L1 is at most as old as the last grid barrier (its acquire invalidates L1), and
+// within a phase distances only fall: an old one is too high, so the test may
+// let a candidate pass that the atomicMin then turns down, and never the reverse.
+// Measured on a B200, kernel time: RMAT scale 16 Bellman-Ford 329 -> 231 us
+// (three sources), scale 18 640 -> 380 us, scale 21 4.6 -> 2.4 ms, scale 23 13.7 ->
+// 8.8 ms; scale 23 learned 2.53 -> 2.17 ms.
+//
+// The loads from L1 go first, all of them: a lane's other load is to the same
+// register and waits for them (each pair in turn took 246 us at scale 16).
+template <int N>
+__device__ __forceinline__ void gather_near(const unsigned long long *dist, const int (&v)[N], const bool (&ok)[N], int near_rows,
+                                            unsigned long long (&out)[N])
+{
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        out[j] = 0;
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.global.ca.b64 %0, [%1];\n}"
+                     : "+l"(out[j])
+                     : "l"(dist + v[j]), "r"((unsigned)(ok[j] && v[j] < near_rows)));
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q ld.global.cg.b64 %0, [%1];\n}"
+                     : "+l"(out[j])
+                     : "l"(dist + v[j]), "r"((unsigned)(ok[j] && v[j] >= near_rows)));
+}
+
+// Which rows that is: all of a graph whose distances fit in the L1 caches some
+// times over (RMAT scale 16: 231 us, 246 with only 8192; scale 18: 380 and 400),
+// otherwise the first ones, since the rest only wash them out (scale 23 learned:
+// 2.25 ms with all, 2.17 with 8192, the same with 2048 to 32768; a uniform graph
+// of 1M vertices 2.19 and 2.14).  The teams of a batch have distances of their
+// own each, whose hot lines lie in different slices, and share the L1s: 512
+// queries on 64 graphs took 4.60 ms without, 4.60 with all and 4.79 with 8192,
+// 32 queries at scale 21 7.55, 7.71 and 7.59.  They don't use it.
+constexpr int32_t kNearAll = 1 << 19, kNearRows = 8192;
+
 __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p)
 {
     unsigned v;
@@ -549,7 +592,7 @@ constexpr int kBuCoop = TRAV_BU_COOP;
 #endif
 // Independent edges per lane per round of a relaxation loop.  More edges in
 // flight hide more latency but cost registers.  With the atomics deferred
-// (SsspPush), SSSP's 64-register budget (4 CTAs per SM) holds 3 without
+// (SsspVisit), SSSP's 64-register budget (4 CTAs per SM) holds 3 without
 // spilling; at s23 a batch of 128 queries ran 8% faster with 3 than with 2,
 // and 4 gained nothing more.  5 CTAs per SM (48 registers) spill and lose 50%.
 constexpr int kBatchBfs = TRAV_KBATCH_BFS, kBatchSssp = TRAV_KBATCH_SSSP;
@@ -581,7 +624,7 @@ struct WarpStage {
     float tdu[32];
 };
 
-// Deferred SSSP relaxations of one warp (see SsspPush): fewer than 32 kept
+// Deferred SSSP relaxations of one warp (see SsspVisit): fewer than 32 kept
 // between batches, plus up to 32 per edge of a lane's batch.
 constexpr int kWDefer = 32 + 32 * kBatchSssp;
 // Where a drain takes a candidate's row-class flags from: the gathered
@@ -1026,7 +1069,8 @@ __device__ __forceinline__ unsigned row_class(const TravArgs &a, int v)
 // (pull rounds): the row's owner is the target, and each in-edge u -> owner
 // gives the candidate fl(d(u) + w).  Both feed the same deferred atomics and
 // push decisions; a pull candidate is just a relaxation of the edge u -> owner.
-template <bool kPull>
+// kNear: gathered distances of the first rows may come from L1 (see gather_near).
+template <bool kPull, bool kNear>
 struct SsspVisit {
     static constexpr int kBatch = kBatchSssp;
     const TravArgs *a;
@@ -1037,6 +1081,21 @@ struct SsspVisit {
     float hold_above = INFINITY;  // light rounds: long rows above this distance wait (see expand_frontier)
 
     __device__ __forceinline__ float begin(int u) const { return dist_of(__ldcg(&a->dist[u])); }
+    __device__ __forceinline__ void gather(const int (&v)[kBatch], const bool (&ok)[kBatch], unsigned long long (&cur)[kBatch]) const
+    {
+        if (kNear && a->near_rows >= a->V) {
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) {
+                cur[j] = 0ull;
+                if (ok[j]) asm volatile("ld.global.ca.b64 %0, [%1];" : "=l"(cur[j]) : "l"(a->dist + v[j]));
+            }
+        } else if (kNear) {
+            gather_near(a->dist, v, ok, a->near_rows, cur);
+        } else {
+#pragma unroll
+            for (int j = 0; j < kBatch; j++) cur[j] = ok[j] ? ld_gather(&a->dist[v[j]]) : 0ull;
+        }
+    }
     __device__ __forceinline__ bool hold(float du) const { return du > hold_above; }
 
     // Queue a held vertex for the next round without a new distance: stamp its
@@ -1092,8 +1151,10 @@ struct SsspVisit {
                 w[j] = ok[j] ? ld_stream(&a->in_w[e[j]]) : 0.0f;
             }
             float nd[kBatch];
+            unsigned long long cur[kBatch];
+            gather(v, ok, cur);
 #pragma unroll
-            for (int j = 0; j < kBatch; j++) nd[j] = ok[j] ? dist_of(ld_gather(&a->dist[v[j]])) : 0.0f;
+            for (int j = 0; j < kBatch; j++) nd[j] = dist_of(cur[j]);
             DeferStage *d = p.d;
 #if TRAV_PULL_REDUCE
             // Lane k of batch j holds edge base + 32 j + k, so for each j the
@@ -1163,8 +1224,7 @@ struct SsspVisit {
         unsigned long long cur[kBatch];
 #pragma unroll
         for (int j = 0; j < kBatch; j++) nd[j] = ok[j] ? __fadd_rn(du[j], w[j]) : 0.0f;  // one rounded add, as sssp.hpp:56
-#pragma unroll
-        for (int j = 0; j < kBatch; j++) cur[j] = ok[j] ? ld_gather(&a->dist[v[j]]) : 0ull;
+        gather(v, ok, cur);
         DeferStage *d = p.d;
 #pragma unroll
         for (int j = 0; j < kBatch; j++) {
@@ -1239,8 +1299,6 @@ struct SsspVisit {
     }
 };
 
-using SsspPush = SsspVisit<false>;
-using SsspPull = SsspVisit<true>;
 
 __device__ __forceinline__ void init_counters(CtaCounters &cc)
 {
@@ -1579,14 +1637,16 @@ __global__ void __launch_bounds__(kBlock, TRAV_BFS_MIN_BLOCKS) bfs_persistent(Tr
 // in x and not below x for w >= 0.
 //
 // Pushes are deduplicated by the round stamps of the distance words (see
-// SsspPush): round ids are phase indices, so the initial words (round 0) are
+// SsspVisit): round ids are phase indices, so the initial words (round 0) are
 // older than every buffer.  A bucket opening pushes from the far pile without
 // lowering a distance, so it stamps each vertex it pushes with its own round
 // (an atomicMax that keeps the distance: nothing lowers distances in that
 // phase).
-template <bool kResume>
+template <bool kResume, bool kNear>
 __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, DeferStage *defer, int ph0)
 {
+    using SsspPush = SsspVisit<false, kNear>;
+    using SsspPull = SsspVisit<true, kNear>;
     SlotView &s_view = sh.view;
     PhaseLog lg;
     lg.leader = (int)blockIdx.x == a.cta0 && threadIdx.x == 0;
@@ -1852,7 +1912,7 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
                 const unsigned cls = (unsigned)dv & kClsMask;
                 const float d = dist_of(dv);
                 const bool in_bucket = valid && d >= told && d < thr;
-                // the pile holds each vertex once (see SsspPush), so every entry is pushed on
+                // the pile holds each vertex once (see SsspVisit), so every entry is pushed on
                 const bool light = in_bucket && (cls & kClsLight);
                 const bool heavy = in_bucket && (cls & kClsHeavy);
                 const bool keep = valid && d >= thr;
@@ -1897,7 +1957,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) sssp_persistent(
     __shared__ QueryShared sh;
     __shared__ DeferStage defer[kWarps];
     init_barrier();
-    sssp_query<kResume>(a, sh, defer, 0);
+    sssp_query<kResume, true>(a, sh, defer, 0);
 }
 
 // ------------------------------------------------------------ batch kernel
@@ -1999,7 +2059,7 @@ __global__ void __launch_bounds__(kBlock, TRAV_SSSP_MIN_BLOCKS) batch_persistent
             a.mean_w = q.mean_w;
             a.max_deg = q.max_deg;
             a.out_kind = 1;
-            ph = sssp_query<false>(a, sh, defer, ph);
+            ph = sssp_query<false, false>(a, sh, defer, ph);
         }
         if (ph < 0) return;
         if (b.done) __threadfence_system();  // this thread's results, before the next dispatch barrier
@@ -2456,6 +2516,7 @@ static TravArgs make_args(const DevGraph &g, Workspace *ws)
     a.timeout_ns = ws->timeout_ns ? ws->timeout_ns : kDefaultTimeoutNs;
     a.mean_w = g.mean_w;
     a.max_deg = g.max_out_degree;
+    a.near_rows = g.V <= kNearAll ? g.V : kNearRows;
     a.cta0 = 0;
     a.ctas = 0;  // set at launch
     a.small_deg = ws->small_deg;
