@@ -1,4 +1,4 @@
-"""SSSP gathers of distances through L1: graphs around the sizes at which all rows, or only the first ones, are read
+"""Gathers of distances (SSSP) and of visited bits (BFS) through L1: graphs around the sizes at which all rows, or only the first ones, are read
 there, with hubs that many edges improve at once.  Distances equal the oracle bit for bit, also when one handle answers
 queries from different sources one after the other (an old distance must never outlive its query) and when one launch
 answers them in turn."""
@@ -36,6 +36,10 @@ def test_distances_around_the_limits(V, E):
                 assert np.array_equal(g.sssp([x], delta=delta)[0].view(np.uint32), ref), (delta, x)
         both = g.sssp(srcs, delta=delta).view(np.uint32)
         assert np.array_equal(both[0], want[0]) and np.array_equal(both[1], want[1])
+    levels = [O.bfs_levels(V, s, d, x, csr_arrays=csr) for x in srcs]
+    for force in (0, -1, 0):
+        for x, ref in zip(srcs, levels):
+            assert np.array_equal(g.bfs([x], force_direction=force)[0], ref), (force, x)
     g.set_grid(1, 5)
     assert np.array_equal(g.sssp([srcs[0]], delta=0.05)[0].view(np.uint32), want[0])
     g.set_grid(1, 0)
