@@ -16,7 +16,7 @@
 // bit says that they matter.
 //
 // Measured, whole calls on a B200: bfs_wrapper on RMAT scale 20, edge factor 16
-// 27.8 -> 0.38 ms; init + bellman_ford_wrapper on 300,007 vertices, 4.8 M edges
+// 27.8 -> 0.33 ms; init + bellman_ford_wrapper on 300,007 vertices, 4.8 M edges
 // 22-28 -> 0.54 ms (before: CSR build, then bfs_persistent / sssp_persistent).
 //
 // A graph whose answer needs many sweeps (long paths) is better served by the
@@ -154,12 +154,22 @@ __device__ __forceinline__ void check_edges(const SweepArgs &a)
 
 // Result of sweep k once its barrier has passed: 0 = nothing changed.  Entry
 // k + 2 of the ring was last read after sweep k - 2's barrier.
-__device__ __forceinline__ void publish(const SweepArgs &a, int k, bool changed)
+__device__ __forceinline__ bool publish(const SweepArgs &a, int k, bool changed)
 {
     const int any = __syncthreads_or(changed);
     if (threadIdx.x == 0) {
         if (any) *reinterpret_cast<volatile int *>(&a.ctl->changed[k & 3]) = 1;
         if (blockIdx.x == 0) *reinterpret_cast<volatile int *>(&a.ctl->changed[(k + 2) & 3]) = 0;
+    }
+    return any;
+}
+
+// Add a CTA's copy of a bitmap to the one in memory.
+__device__ __forceinline__ void merge_bits(unsigned *g, const unsigned *copy, int W)
+{
+    for (int w = threadIdx.x; w < W; w += kSweepThreads) {
+        const unsigned x = copy[w] & ~__ldcg(&g[w]);
+        if (x) atomicOr(&g[w], x);
     }
 }
 
@@ -172,6 +182,12 @@ __device__ __forceinline__ int changed_in(const SweepArgs &a, int k)
 // reached or outside the tree, which no edge may reach.  An edge matters when
 // its target is still open and its source is reached; late sweeps find almost
 // every target closed and read 4 bytes an edge.
+//
+// With the bitmaps in shared memory a CTA marks what it finds there, and takes
+// its copy to memory once a sweep, a word an atomic and 32 consecutive words a
+// warp.  (A global atomic for every vertex that a CTA finds was up to one per
+// edge in the sweep that reaches most vertices, each waited for.)  RMAT scale 20,
+// edge factor 16, whole call: 0.39 -> 0.33 ms.
 template <bool kMask, bool kSmem>
 __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
 {
@@ -230,19 +246,17 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
                 for (int j = 0; j < 4; j++) {
                     if (!((open[u] >> j) & 1u) || !test(r, fv[j])) continue;
                     const unsigned bit = 1u << (tv[j] & 31);
-                    // the CTA's own copy first: one global atomic per vertex and CTA
-                    if (kSmem) {
-                        const unsigned old = atomicOr(&r[tv[j] >> 5], bit);
-                        if (kMask) atomicOr(&c[tv[j] >> 5], bit);
-                        if (old & bit) continue;
-                    }
-                    const unsigned old = atomicOr(&gr[tv[j] >> 5], bit);
-                    if (kMask) atomicOr(&gc[tv[j] >> 5], bit);
+                    // in the CTA's own copy (merge_bits takes it to memory)
+                    const unsigned old = atomicOr(&r[tv[j] >> 5], bit);
+                    if (kMask) atomicOr(&c[tv[j] >> 5], bit);
                     if (!(old & bit)) changed = true;
                 }
             }
         }
-        publish(a, k, changed);
+        if (publish(a, k, changed) && kSmem) {
+            merge_bits(gr, r, a.W);
+            if (kMask) merge_bits(gc, c, a.W);
+        }
         if (!sweep_sync(a, phase++)) return;
         done = !changed_in(a, k);
     }
