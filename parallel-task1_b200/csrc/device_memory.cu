@@ -3,11 +3,13 @@
 // cudaMalloc and cudaFree of a few megabytes take 0.3 ms each on a B200, a
 // stream 0.1 ms; a call that builds a graph handle for one query, as the
 // reference's callers do, made some 35 allocations and spent 20 of its 27 ms
-// there.  Arrays that live together share one allocation (DevSlab), and freed blocks stay here for the next allocation of about their
-// size, up to kKeepBytes per device (0.15% of the memory); the oldest go first
-// when the bound is reached, and all of them when an allocation fails.
-// Measured: a graph built from 4.2 M host edges, one BFS and one SSSP, 31 -> 7.8
-// ms; the optimisation pass on 8.4 M edges 10.9 -> 5.4 ms.
+// there.  Arrays that live together share one allocation (DevSlab), and freed
+// blocks stay here for the next allocation of about their size, up to kKeepBytes
+// per device (0.6% of the memory); the oldest go first when the bound is
+// reached, and all of them when an allocation fails.
+// Measured: a graph built from 4.2 M host edges, one BFS and one SSSP, 31 -> 6.0
+// ms; the optimisation pass on 8.4 M edges 10.9 -> 2.7 ms (8.4 and 5.0 ms with a
+// bound of 256 MB, which the blocks of these two calls exceed).
 // Blocks larger than the bound come from cudaMalloc and go back to it.
 //
 // A block is idle before it is kept (dev_free waits for the device, as
@@ -25,7 +27,7 @@
 namespace trav {
 namespace {
 
-constexpr size_t kKeepBytes = size_t(256) << 20;
+constexpr size_t kKeepBytes = size_t(1024) << 20;
 constexpr size_t kKeepStreams = 8;
 
 struct Block {
