@@ -188,9 +188,10 @@ int trav_bfs_el(const int32_t *src, const int32_t *dst, int32_t vertices, int64_
  * src[e] -> dst[e] whose two ends lie in the same tree (trees[src] ==
  * trees[dst]); visited[v] = 1 for every vertex reached, else 0 (C++ bool
  * layout).  All arrays, pivot included, are device memory, as in the
- * reference; the backward sweep passes dst as src.  Runs on this library's
- * BFS kernels (the tree restriction is a vertex mask: only vertices of the
- * pivot's tree are ever reached).  Synchronous. */
+ * reference; the backward sweep passes dst as src.  Sweeps the edge list on the
+ * device; a graph that needs many sweeps goes to this library's BFS kernels
+ * (the tree restriction is a vertex mask: only vertices of the pivot's tree are
+ * ever reached).  Synchronous. */
 int trav_reach_el_masked(const int32_t *src, const int32_t *dst, int32_t vertices, int64_t edges,
                          const int32_t *pivot, const int32_t *trees, uint8_t *visited);
 
