@@ -16,8 +16,8 @@
 // bit says that they matter.
 //
 // Measured, whole calls on a B200: bfs_wrapper on RMAT scale 20, edge factor 16
-// 27.8 -> 0.33 ms; init + bellman_ford_wrapper on 300,007 vertices, 4.8 M edges
-// 22-28 -> 0.54 ms (before: CSR build, then bfs_persistent / sssp_persistent).
+// 27.8 -> 0.29 ms; init + bellman_ford_wrapper on 300,007 vertices, 4.8 M edges
+// 22-28 -> 0.48 ms (before: CSR build, then bfs_persistent / sssp_persistent).
 //
 // A graph whose answer needs many sweeps (long paths) is better served by the
 // CSR kernels, whose steps touch the frontier only: after kMaxSweeps sweeps
@@ -108,12 +108,18 @@ __device__ bool sweep_sync(const SweepArgs &a, int phase)
     return s_ok != 0;
 }
 
-__device__ __forceinline__ int4 ld4(const int32_t *p) { return __ldcs(reinterpret_cast<const int4 *>(p)); }
-
-// The four edges at e (e % 4 == 0) of an array; entries at or past E read as `fill`.
+// The four edges at e (e % 4 == 0) of an array; entries at or past E read as
+// `fill`.  kAgain: the next sweep reads them again, so they may stay in L2
+// (the others are marked to leave first).  The targets of a reachability sweep,
+// RMAT scale 20: 302 -> 289 us a call; all of a Bellman-Ford sweep's, 300,007
+// vertices, 4.8 M edges: 548 -> 483 us.
+template <bool kAgain = false>
 __device__ __forceinline__ int4 edge4(const int32_t *p, unsigned e, unsigned E, int vec, int fill)
 {
-    if (vec && e + 4 <= E) return ld4(p + e);
+    if (vec && e + 4 <= E) {
+        const int4 *q = reinterpret_cast<const int4 *>(p + e);
+        return kAgain ? __ldg(q) : __ldcs(q);
+    }
     int4 r;
     r.x = e < E ? __ldcs(p + e) : fill;
     r.y = e + 1 < E ? __ldcs(p + e + 1) : fill;
@@ -152,6 +158,31 @@ __device__ __forceinline__ void check_edges(const SweepArgs &a)
     if (flag && (threadIdx.x & 31) == 0) atomicOr(&a.ctl->bad, flag);
 }
 
+// The same for reachability with the bitmap in shared memory, as a sweep: an
+// edge whose ends are in range and whose source is reached marks its target.
+// It reads both ends of every edge, as the first sweep would again (RMAT scale
+// 20: 337 -> 302 us a call).
+__device__ __forceinline__ bool check_and_mark(const SweepArgs &a, unsigned *reached)
+{
+    const unsigned E = (unsigned)a.E, V = (unsigned)a.V, step = gridDim.x * kSweepThreads * 4;
+    int flag = 0;
+    bool marked = false;
+    for (unsigned e = (blockIdx.x * kSweepThreads + threadIdx.x) * 4; e < E; e += step) {
+        const int4 f = edge4(a.src, e, E, a.vec, 0), t = edge4(a.dst, e, E, a.vec, 0);
+        flag |= check_ids(f, a.V) | check_ids(t, a.V);
+        const int fv[4] = {f.x, f.y, f.z, f.w}, tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (e + j >= E || (unsigned)fv[j] >= V || (unsigned)tv[j] >= V || !test(reached, fv[j])) continue;
+            atomicOr(&reached[tv[j] >> 5], 1u << (tv[j] & 31));
+            marked = true;
+        }
+    }
+    flag = __reduce_or_sync(kAll, flag);
+    if (flag && (threadIdx.x & 31) == 0) atomicOr(&a.ctl->bad, flag);
+    return marked;
+}
+
 // Result of sweep k once its barrier has passed: 0 = nothing changed.  Entry
 // k + 2 of the ring was last read after sweep k - 2's barrier.
 __device__ __forceinline__ bool publish(const SweepArgs &a, int k, bool changed)
@@ -178,7 +209,7 @@ __device__ __forceinline__ int changed_in(const SweepArgs &a, int k)
     return *reinterpret_cast<volatile int *>(&a.ctl->changed[k & 3]);
 }
 
-// Reachability.  bits[0]: vertices reached; bits[1] (kMask only): vertices
+// Reachability.  bits[0] (clear at first): vertices reached; bits[1] (kMask only): vertices
 // reached or outside the tree, which no edge may reach.  An edge matters when
 // its target is still open and its source is reached; late sweeps find almost
 // every target closed and read 4 bytes an edge.
@@ -187,7 +218,7 @@ __device__ __forceinline__ int changed_in(const SweepArgs &a, int k)
 // its copy to memory once a sweep, a word an atomic and 32 consecutive words a
 // warp.  (A global atomic for every vertex that a CTA finds was up to one per
 // edge in the sweep that reaches most vertices, each waited for.)  RMAT scale 20,
-// edge factor 16, whole call: 0.39 -> 0.33 ms.
+// edge factor 16, whole call: 0.39 -> 0.34 ms.
 template <bool kMask, bool kSmem>
 __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
 {
@@ -195,8 +226,16 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
     const int gtid = blockIdx.x * kSweepThreads + threadIdx.x, nth = gridDim.x * kSweepThreads;
     unsigned *const gr = a.bits[0], *const gc = kMask ? a.bits[1] : a.bits[0];
     unsigned *const r = kSmem ? sm : gr, *const c = kMask ? (kSmem ? sm + a.W : gc) : r;
-    check_edges(a);
     const int s = a.source;
+    if (!kMask && kSmem) {
+        // gr is clear
+        for (int w = threadIdx.x; w < a.W; w += kSweepThreads) sm[w] = w == (s >> 5) ? 1u << (s & 31) : 0u;
+        __syncthreads();
+        const bool marked = check_and_mark(a, sm);
+        if (__syncthreads_or(marked) || blockIdx.x == 0) merge_bits(gr, sm, a.W);
+    } else {
+        check_edges(a);
+    }
     if (kMask) {
         for (int w = gtid >> 5; w < a.W; w += nth >> 5) {
             const int v = w * 32 + (int)(threadIdx.x & 31);
@@ -206,7 +245,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
                 gc[w] = m;
             }
         }
-    } else {
+    } else if (!kSmem) {
         for (int w = gtid; w < a.W; w += nth) gr[w] = w == (s >> 5) ? 1u << (s & 31) : 0u;
     }
     int phase = 0;
@@ -231,7 +270,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
 #pragma unroll
             for (int u = 0; u < kU; u++) {
                 const unsigned e = e0 + u * step;
-                t[u] = e < E ? edge4(a.dst, e, E, a.vec, s) : make_int4(s, s, s, s);  // the source is closed
+                t[u] = e < E ? edge4<true>(a.dst, e, E, a.vec, s) : make_int4(s, s, s, s);  // the source is closed
             }
 #pragma unroll
             for (int u = 0; u < kU; u++)
@@ -321,7 +360,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_bellman_ford_kernel(Sweep
 #pragma unroll
             for (int u = 0; u < kU; u++) {
                 const unsigned e = e0 + u * step;
-                f[u] = e < E ? edge4(a.src, e, E, a.vec, -1) : make_int4(-1, -1, -1, -1);
+                f[u] = e < E ? edge4<true>(a.src, e, E, a.vec, -1) : make_int4(-1, -1, -1, -1);
             }
 #pragma unroll
             for (int u = 0; u < kU; u++)
@@ -331,8 +370,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_bellman_ford_kernel(Sweep
             for (int u = 0; u < kU; u++) {
                 if (!on[u]) continue;
                 const unsigned e = e0 + u * step;
-                const int4 t = edge4(a.dst, e, E, a.vec, 0);
-                const int4 wt = edge4(reinterpret_cast<const int32_t *>(a.w), e, E, a.vec, 0);
+                const int4 t = edge4<true>(a.dst, e, E, a.vec, 0);
+                const int4 wt = edge4<true>(reinterpret_cast<const int32_t *>(a.w), e, E, a.vec, 0);
                 const int fv[4] = {f[u].x, f[u].y, f[u].z, f[u].w}, tv[4] = {t.x, t.y, t.z, t.w};
                 const int wv[4] = {wt.x, wt.y, wt.z, wt.w};
                 float nd[4], od[4];
@@ -403,7 +442,7 @@ int run_sweeps(SweepArgs a, int maps, int copied, const void *fn_smem, const voi
     int64_t ctas = (a.E + kCtaEdges - 1) / kCtaEdges;
     if (ctas < 1) ctas = 1;
     if (ctas > sms) ctas = sms;  // one CTA of 1024 threads per SM
-    TRY_CUDA(cudaMemsetAsync(a.ctl, 0, sizeof(SweepCtl), st));
+    TRY_CUDA(cudaMemsetAsync(mem.p, 0, 256 + map_bytes, st));  // ctl and the first bitmap
     void *params[] = {&a};
     TRY_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)ctas), dim3(kSweepThreads), params, fits ? smem : 0, st));
     SweepCtl h;
