@@ -527,7 +527,7 @@ int trav_el_optimize(int32_t *src, int32_t *dst, float *w, int32_t vertices, int
         s = ds.p, d = dd.p, ww = dw.p;
     }
     TRY(validate_edges(vertices, edges, s, d, ww, 0));
-    TRY(el_optimize_device(s, d, ww, edges, segment, edges_out, 0));
+    TRY(el_optimize_device(s, d, ww, vertices, edges, segment, edges_out, 0));
     if (mem == TRAV_MEM_HOST && *edges_out > 0) {
         const size_t n = (size_t)*edges_out;
         TRY_CUDA(cudaMemcpy(src, s, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));

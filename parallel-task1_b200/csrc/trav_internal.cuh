@@ -348,7 +348,7 @@ int el_bellman_ford_sweeps(const int32_t *src, const int32_t *dst, const float *
                            cudaStream_t st, bool *done);
 
 // el_optimize.cu
-int el_optimize_device(int32_t *src, int32_t *dst, float *w, int64_t E, int32_t segment, int64_t *E_out,
+int el_optimize_device(int32_t *src, int32_t *dst, float *w, int32_t V, int64_t E, int32_t segment, int64_t *E_out,
                        cudaStream_t st);
 int el_transactions_device(const int32_t *src, const int32_t *dst, int64_t E, int32_t elem, int64_t *count,
                            cudaStream_t st);
