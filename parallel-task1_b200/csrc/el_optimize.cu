@@ -7,7 +7,7 @@
 //   reorder_edges_for_cache                 :122-166 group by (src / segment, dst / segment)
 //   check_gpu_memory_transactions_count     :229-266 distinct 128-byte segments per warp of 32 edges
 //
-// The sorts are stable radix sorts (weight bits, then the 64-bit (src, dst)
+// The sorts are stable radix sorts (weight bits, then the (src, dst)
 // key, then the segment key), so the order inside a segment pair -- which the
 // reference's std::sort leaves unspecified -- is the (src, dst, weight) order.
 #include <cuda_runtime.h>
