@@ -101,9 +101,9 @@ TeamLayout team_layout(const trav_batch *b)
 int release_teams(trav_batch *b)
 {
     TRY_CUDA(cudaStreamSynchronize(b->st));
-    dev_free(b->team_mem);
-    dev_free(b->d_teams);
-    dev_free(b->ctl);
+    dev_free(b->team_mem, b->st);
+    dev_free(b->d_teams, b->st);
+    dev_free(b->ctl, b->st);
     b->team_mem = nullptr;
     b->d_teams = nullptr;
     b->ctl = nullptr;
@@ -332,7 +332,7 @@ int upload_queries(trav_batch *b, const trav_query *qs, int32_t n, int smooth_ta
     TRY(build_queries(b, qs, n, &d, smooth_tail));
     if (n > b->q_cap) {
         TRY_CUDA(cudaStreamSynchronize(b->st));
-        dev_free(b->d_q);
+        dev_free(b->d_q, b->st);
         b->d_q = nullptr;
         b->q_cap = 0;
         TRY_CUDA(dev_malloc(&b->d_q, sizeof(BatchQuery) * (size_t)n));
@@ -423,14 +423,14 @@ void trav_batch_free(trav_batch *b)
     if (!b) return;
     cudaSetDevice(b->device);
     if (b->st) cudaStreamSynchronize(b->st);
-    dev_free(b->team_mem);
-    dev_free(b->d_teams);
-    dev_free(b->ctl);
-    dev_free(b->d_q);
-    dev_free(b->d_next);
-    for (auto &kv : b->light) light_rows_free(&kv.second);
+    dev_free(b->team_mem, b->st);
+    dev_free(b->d_teams, b->st);
+    dev_free(b->ctl, b->st);
+    dev_free(b->d_q, b->st);
+    dev_free(b->d_next, b->st);
+    for (auto &kv : b->light) light_rows_free(&kv.second, b->st);
     if (b->cst) cudaStreamSynchronize(b->cst);
-    dev_free(b->staging);
+    dev_free(b->staging, b->st);
     cudaFreeHost(b->done);
     stream_put(b->cst);
     if (b->ev0) cudaEventDestroy(b->ev0);
@@ -470,7 +470,7 @@ int trav_batch_run_host(trav_batch *b, const trav_query *queries, int32_t n, int
         at[(size_t)i + 1] = at[(size_t)i] + 4 * (size_t)b->graphs[(size_t)queries[i].graph]->g.V;
     if (at[(size_t)n] > b->staging_bytes) {
         if (b->cst) TRY_CUDA(cudaStreamSynchronize(b->cst));
-        dev_free(b->staging);
+        dev_free(b->staging, b->st);
         b->staging = nullptr;
         b->staging_bytes = 0;
         // Team scratch is sized to the free memory when it is allocated, so on

@@ -97,18 +97,18 @@ void destroy(trav_graph *h)
     cudaSetDevice(h->device);
     if (h->st) cudaStreamSynchronize(h->st);
     if (h->cst) cudaStreamSynchronize(h->cst);
-    free_graph(&h->g);
-    workspace_free(&h->ws);
+    free_graph(&h->g, h->st);
+    workspace_free(&h->ws, h->st);
     for (int b = 0; b < 2; b++) {
-        dev_free(h->staging[b]);
+        dev_free(h->staging[b], h->cst);
         if (h->done[b]) cudaEventDestroy(h->done[b]);
         if (h->copied[b]) cudaEventDestroy(h->copied[b]);
     }
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     for (auto &c : h->cap)
         if (c.exec) cudaGraphExecDestroy(c.exec);
-    dev_free(h->mlp[0]);
-    dev_free(h->mlp[1]);
+    dev_free(h->mlp[0], nullptr);  // written on the legacy stream; its readers have been waited for
+    dev_free(h->mlp[1], nullptr);
     stream_put(h->cst);
     stream_put(h->own_st);
     delete h;
@@ -248,10 +248,13 @@ int run_batch(trav_graph *g, int kind, const int32_t *sources, int32_t n, const 
     return TRAV_OK;
 }
 
+// Device array that a call works on in stream st.
 template <class T>
 struct DevTmp {
     T *p = nullptr;
-    ~DevTmp() { if (p) dev_free(p); }
+    cudaStream_t st;
+    explicit DevTmp(cudaStream_t s) : st(s) {}
+    ~DevTmp() { dev_free(p, st); }
 };
 
 int check_sources(const trav_graph *h, const int32_t *sources, int32_t n)
@@ -293,8 +296,8 @@ int trav_graph_from_edges(int32_t vertices, int64_t edges, const int32_t *src, c
     trav_graph *h = nullptr;
     TRY(new_handle(&h));
     std::unique_ptr<trav_graph, void (*)(trav_graph *)> guard(h, destroy);
-    DevTmp<int32_t> ds, dd;
-    DevTmp<float> dw;
+    DevTmp<int32_t> ds(h->st), dd(h->st);
+    DevTmp<float> dw(h->st);
     const int32_t *ps = src, *pd = dst;
     const float *pw = w;
     if (mem == TRAV_MEM_HOST && edges > 0) {
@@ -333,8 +336,8 @@ int trav_graph_rmat(int32_t scale, int32_t avg, int32_t a, int32_t b, int32_t c,
     trav_graph *h = nullptr;
     TRY(new_handle(&h));
     std::unique_ptr<trav_graph, void (*)(trav_graph *)> guard(h, destroy);
-    DevTmp<int32_t> ds, dd;
-    DevTmp<float> dw;
+    DevTmp<int32_t> ds(h->st), dd(h->st);
+    DevTmp<float> dw(h->st);
     int32_t *ps = src, *pd = dst;
     float *pw = w;
     if (!src) {
@@ -512,8 +515,8 @@ int trav_el_optimize(int32_t *src, int32_t *dst, float *w, int32_t vertices, int
     if (mem == TRAV_MEM_DEVICE && (!is_device_ptr(src) || !is_device_ptr(dst) || !is_device_ptr(w)))
         return bad("src, dst and w must be device arrays (mem = TRAV_MEM_DEVICE)");
     TRY_CUDA(cudaDeviceSynchronize());
-    DevTmp<int32_t> ds, dd;
-    DevTmp<float> dw;
+    DevTmp<int32_t> ds(nullptr), dd(nullptr);
+    DevTmp<float> dw(nullptr);
     int32_t *s = src, *d = dst;
     float *ww = w;
     const size_t bi = sizeof(int32_t) * (size_t)edges, bf = sizeof(float) * (size_t)edges;
@@ -550,7 +553,7 @@ int trav_el_gpu_transactions(const int32_t *src, const int32_t *dst, int32_t ver
     if (mem == TRAV_MEM_DEVICE && (!is_device_ptr(src) || !is_device_ptr(dst)))
         return bad("src and dst must be device arrays (mem = TRAV_MEM_DEVICE)");
     TRY_CUDA(cudaDeviceSynchronize());
-    DevTmp<int32_t> ds, dd;
+    DevTmp<int32_t> ds(nullptr), dd(nullptr);
     const int32_t *s = src, *d = dst;
     if (mem == TRAV_MEM_HOST) {
         const size_t bi = sizeof(int32_t) * (size_t)edges;
@@ -610,7 +613,7 @@ int trav_set_plan(trav_graph *g, int32_t kind, const uint8_t *plan, int32_t n)
     if (n < 0 || (n > 0 && !plan)) return bad("plan must hold n >= 0 entries");
     TRY_CUDA(cudaSetDevice(g->device));
     TRY_CUDA(cudaStreamSynchronize(g->st));
-    dev_free(g->ws.plan[kind]);
+    dev_free(g->ws.plan[kind], nullptr);  // written on the legacy stream
     g->ws.plan[kind] = nullptr;
     g->ws.plan_len[kind] = 0;
     if (n == 0) return TRAV_OK;
@@ -834,7 +837,7 @@ int trav_reach_el_masked(const int32_t *src, const int32_t *dst, int32_t vertice
     if (done) return TRAV_OK;
     TRY(build_graph_device(vertices, edges, src, dst, nullptr, h->st, &h->g));
     TRY(workspace_ensure(&h->ws, h->g, 1, h->st));
-    DevTmp<int32_t> color;
+    DevTmp<int32_t> color(h->st);
     TRY_CUDA(dev_malloc(&color.p, sizeof(int32_t) * (size_t)vertices));
     permute_color_kernel<<<(vertices + 255) / 256 < 4096 ? (vertices + 255) / 256 : 4096, 256, 0, h->st>>>(
         color.p, trees, h->g.old_of_new, vertices);

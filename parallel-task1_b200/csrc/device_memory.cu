@@ -12,8 +12,10 @@
 // bound of 256 MB, which the blocks of these two calls exceed).
 // Blocks larger than the bound come from cudaMalloc and go back to it.
 //
-// A block is idle before it is kept (dev_free waits for the device, as
-// cudaFree does), so its next owner may use it on any stream.
+// A block is idle before it is kept (dev_free waits for the stream of its last
+// work), so its next owner may use it on any stream.  A wait for the whole device
+// would do the same, but CUDA refuses one while any of its streams is captured,
+// and the capture, another thread's perhaps, is lost.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -124,7 +126,7 @@ cudaError_t dev_malloc_bytes(void **p, size_t bytes)
     return cudaSuccess;
 }
 
-void dev_free(void *p)
+void dev_free(void *p, cudaStream_t st)
 {
     if (!p) return;
     Block b{p, 0, -1};
@@ -143,9 +145,10 @@ void dev_free(void *p)
     // nothing may still read or write the block when it is handed on
     const int cur = current_device();
     if (cur != b.device) cudaSetDevice(b.device);
-    const cudaError_t e = cudaDeviceSynchronize();
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (cur != b.device) cudaSetDevice(cur);
     if (e != cudaSuccess) {
+        cudaGetLastError();  // not the caller's next launch's
         cudaFree(p);
         return;
     }

@@ -31,8 +31,10 @@ namespace {
 template <class T>
 struct Buf {
     T *p = nullptr;
+    cudaStream_t st;
+    explicit Buf(cudaStream_t s) : st(s) {}
     cudaError_t alloc(int64_t n) { return dev_malloc((void **)&p, sizeof(T) * (size_t)(n > 0 ? n : 1)); }
-    ~Buf() { if (p) dev_free(p); }
+    ~Buf() { dev_free(p, st); }
 };
 
 int grid_of(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 65535); }
@@ -132,7 +134,7 @@ int el_optimize_device(int32_t *src, int32_t *dst, float *w, int32_t V, int64_t 
 {
     *E_out = 0;
     if (E == 0) return TRAV_OK;
-    DevSlab mem;
+    DevSlab mem(st);
     unsigned *wkey, *wkey2;
     int32_t *idx, *idx2, *s2, *d2;
     unsigned long long *key, *key2;
@@ -197,7 +199,7 @@ int el_transactions_device(const int32_t *src, const int32_t *dst, int64_t E, in
                            cudaStream_t st)
 {
     const int64_t warps = E > 0 ? (E - 1) / 32 : 0;  // the warp holding the last edge is not counted
-    Buf<unsigned long long> tot;
+    Buf<unsigned long long> tot(st);
     TRY_CUDA(tot.alloc(1));
     TRY_CUDA(cudaMemsetAsync(tot.p, 0, sizeof(unsigned long long), st));
     if (warps > 0) {

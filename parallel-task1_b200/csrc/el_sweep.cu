@@ -412,7 +412,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_bellman_ford_kernel(Sweep
 
 struct Scratch {
     void *p = nullptr;
-    ~Scratch() { if (p) dev_free(p); }
+    cudaStream_t st;
+    explicit Scratch(cudaStream_t s) : st(s) {}
+    ~Scratch() { dev_free(p, st); }
 };
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -427,7 +429,7 @@ int run_sweeps(SweepArgs a, int maps, int copied, const void *fn_smem, const voi
     a.vec = aligned16(a.src) && aligned16(a.dst) && aligned16(a.w);
     a.timeout_ns = kDefaultTimeoutNs;
     const size_t map_bytes = (sizeof(unsigned) * (size_t)a.W + 255) & ~(size_t)255;
-    Scratch mem;
+    Scratch mem(st);
     TRY_CUDA(dev_malloc(&mem.p, 256 + map_bytes * (size_t)maps));
     unsigned char *m = static_cast<unsigned char *>(mem.p);
     a.ctl = reinterpret_cast<SweepCtl *>(m);

@@ -212,8 +212,10 @@ __global__ void weight_sum_kernel(int64_t E, const float *__restrict__ w, double
 template <class T>
 struct DBuf {
     T *p = nullptr;
+    cudaStream_t st;
+    explicit DBuf(cudaStream_t s) : st(s) {}
     cudaError_t alloc(int64_t n) { return dev_malloc((void **)&p, sizeof(T) * (size_t)(n > 0 ? n : 1)); }
-    ~DBuf() { dev_free(p); }
+    ~DBuf() { dev_free(p, st); }
 };
 
 #define TRY_CUDA(expr)                                   \
@@ -241,10 +243,10 @@ int rmat_device(int scale, int avg, int a, int b, int c, int d, uint32_t seed, i
     rmat_kernel<<<blocks, threads, 0, st>>>(scale, E, a, b, c, d, seed, gap, spe, d_src, d_dst, d_w);
     TRY_CUDA(cudaGetLastError());
     if (drop_loops) {
-        DBuf<unsigned char> keep;
-        DBuf<int32_t> tmp_i;
-        DBuf<float> tmp_f;
-        DBuf<int64_t> nsel;
+        DBuf<unsigned char> keep(st);
+        DBuf<int32_t> tmp_i(st);
+        DBuf<float> tmp_f(st);
+        DBuf<int64_t> nsel(st);
         TRY_CUDA(keep.alloc(E));
         TRY_CUDA(tmp_i.alloc(E));
         TRY_CUDA(tmp_f.alloc(E));
@@ -252,7 +254,7 @@ int rmat_device(int scale, int avg, int a, int b, int c, int d, uint32_t seed, i
         loop_flags_kernel<<<grid_for(E), 256, 0, st>>>(d_src, d_dst, E, keep.p);
         size_t tb = 0;
         TRY_CUDA(cub::DeviceSelect::Flagged(nullptr, tb, d_src, keep.p, tmp_i.p, nsel.p, E, st));
-        DBuf<unsigned char> temp;
+        DBuf<unsigned char> temp(st);
         TRY_CUDA(temp.alloc((int64_t)tb));
         int64_t n = 0;
         TRY_CUDA(cub::DeviceSelect::Flagged(temp.p, tb, d_src, keep.p, tmp_i.p, nsel.p, E, st));
@@ -274,7 +276,7 @@ int validate_edges(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_
                    cudaStream_t st)
 {
     if (E == 0) return TRAV_OK;
-    DBuf<int> bad;
+    DBuf<int> bad(st);
     TRY_CUDA(bad.alloc(1));
     TRY_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), st));
     validate_kernel<<<grid_for(E), 256, 0, st>>>(V, E, d_src, d_dst, d_w, bad.p);
@@ -288,9 +290,9 @@ int validate_edges(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_
     return TRAV_OK;
 }
 
-void free_graph(DevGraph *g)
+void free_graph(DevGraph *g, cudaStream_t st)
 {
-    dev_free(g->mem);
+    dev_free(g->mem, st);
     *g = DevGraph{};
 }
 
@@ -304,7 +306,7 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
     const unsigned long long mask = (1ull << lv) - 1ull;
 
     // What the handle keeps and what only the build needs: one allocation each.
-    DevSlab keep, tmp;
+    DevSlab keep(st), tmp(st);
     DevGraph g;
     keep.add(&g.out_off, (int64_t)V + 1);
     keep.add(&g.in_off, (int64_t)V + 1);

@@ -169,15 +169,16 @@ struct MlpDev {
     int *y = nullptr;
     ~MlpDev()
     {
-        dev_free(p);
-        dev_free(g);
-        dev_free(m);
-        dev_free(v);
-        dev_free(x);
-        dev_free(partial);
-        dev_free(lpart);
-        dev_free(loss);
-        dev_free(y);
+        // everything here runs on the legacy stream
+        dev_free(p, nullptr);
+        dev_free(g, nullptr);
+        dev_free(m, nullptr);
+        dev_free(v, nullptr);
+        dev_free(x, nullptr);
+        dev_free(partial, nullptr);
+        dev_free(lpart, nullptr);
+        dev_free(loss, nullptr);
+        dev_free(y, nullptr);
     }
 };
 

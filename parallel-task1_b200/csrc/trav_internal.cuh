@@ -279,10 +279,11 @@ bool is_device_ptr(const void *p);
 
 // Every device allocation of the library goes through dev_malloc and back
 // through dev_free (device_memory.cu), which keeps freed blocks for the next
-// call, up to a bound.  When a test armed trav_inject_alloc_failure, the armed
+// call, up to a bound.  dev_free waits for `st`, the stream of the block's last
+// work; work that other streams did on it must have ended.  When a test armed trav_inject_alloc_failure, the armed
 // allocation fails with cudaErrorMemoryAllocation as cudaMalloc would.
 cudaError_t dev_malloc_bytes(void **p, size_t bytes);
-void dev_free(void *p);
+void dev_free(void *p, cudaStream_t st);
 // True when the armed failure falls on this allocation (each array of a DevSlab counts as one).
 bool alloc_failure_due();
 void arm_alloc_failure(int32_t after);
@@ -296,10 +297,12 @@ inline cudaError_t dev_malloc(T **p, size_t bytes)
 }
 
 // Several arrays in one allocation: add() each, then commit().  The slab owns
-// the memory until release() hands it on (to be freed with dev_free).
+// the memory until release() hands it on (to be freed with dev_free); `st` is
+// the stream that works on it.
 class DevSlab {
 public:
-    ~DevSlab() { dev_free(mem_); }
+    explicit DevSlab(cudaStream_t st) : st_(st) {}
+    ~DevSlab() { dev_free(mem_, st_); }
     template <class T>
     void add(T **p, int64_t n)
     {
@@ -328,12 +331,13 @@ private:
     std::vector<Part> parts_;
     size_t bytes_ = 0;
     void *mem_ = nullptr;
+    cudaStream_t st_;
 };
 
 // ingest.cu
 int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_dst, const float *d_w,
                        cudaStream_t st, DevGraph *out);
-void free_graph(DevGraph *g);
+void free_graph(DevGraph *g, cudaStream_t st);
 int rmat_device(int scale, int avg, int a, int b, int c, int d, uint32_t seed, int drop_loops,
                 int32_t *d_src, int32_t *d_dst, float *d_w, int64_t *E_out, cudaStream_t st);
 int validate_edges(int32_t V, int64_t E, const int32_t *d_src, const int32_t *d_dst, const float *d_w,
@@ -355,7 +359,7 @@ int el_transactions_device(const int32_t *src, const int32_t *dst, int64_t E, in
 
 // traverse.cu
 int workspace_ensure(Workspace *ws, const DevGraph &g, int nqueries, cudaStream_t st);
-void workspace_free(Workspace *ws);
+void workspace_free(Workspace *ws, cudaStream_t st);
 // Enqueue one query on st using control block ws->ctl[q] (no host sync).
 // ev0/ev1 (optional) are recorded around the launch.
 // color (new ids, may be nullptr): reach only vertices with color[v] == color_want.
@@ -371,7 +375,7 @@ int check_ctls(const Ctl *ctl, int n, const char *what, cudaStream_t st);  // th
 int count_light(const DevGraph &g, float delta, int32_t *nlight, cudaStream_t st);
 // Build (or rebuild for a new delta) the light rows of g; no-op when lr already holds delta.
 int light_rows_build(const DevGraph &g, float delta, LightRows *lr, cudaStream_t st);
-void light_rows_free(LightRows *lr);
+void light_rows_free(LightRows *lr, cudaStream_t st);
 int query_bytes(const DevGraph &g, Workspace *ws, int q, int kind, int64_t *bytes, int64_t *reached,
                 int64_t *reached_edges, cudaStream_t st);
 int persistent_grid_size(int kind);  // kind 2 = the batch kernel

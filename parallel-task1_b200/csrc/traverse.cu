@@ -2379,11 +2379,11 @@ int count_light(const DevGraph &g, float delta, int32_t *nlight, cudaStream_t st
     return TRAV_OK;
 }
 
-void light_rows_free(LightRows *lr)
+void light_rows_free(LightRows *lr, cudaStream_t st)
 {
-    dev_free(lr->nlight);
-    dev_free(lr->loff);
-    dev_free(lr->ledge);
+    dev_free(lr->nlight, st);
+    dev_free(lr->loff, st);
+    dev_free(lr->ledge, st);
     *lr = LightRows{};
 }
 
@@ -2394,7 +2394,7 @@ void light_rows_free(LightRows *lr)
 int light_rows_build(const DevGraph &g, float delta, LightRows *lr, cudaStream_t st)
 {
     if (lr->delta == delta && lr->nlight) return TRAV_OK;
-    light_rows_free(lr);
+    light_rows_free(lr, st);
     const int32_t V = g.V > 0 ? g.V : 1;
     TRY_CUDA(dev_malloc(&lr->nlight, sizeof(int32_t) * (size_t)V));
     TRY(count_light(g, delta, lr->nlight, st));
@@ -2410,7 +2410,7 @@ int light_rows_build(const DevGraph &g, float delta, LightRows *lr, cudaStream_t
     if (e == cudaSuccess && g.V > 0) e = cudaMemcpyAsync(&last[0], lr->loff + g.V - 1, 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && g.V > 0) e = cudaMemcpyAsync(&last[1], lr->nlight + g.V - 1, 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    dev_free(tmp);
+    dev_free(tmp, st);
     if (e != cudaSuccess) return cuda_fail(e, "light row offsets");
     const int32_t total = last[0] + last[1];
     TRY_CUDA(cudaMemcpyAsync(lr->loff + g.V, &total, sizeof(int32_t), cudaMemcpyHostToDevice, st));
@@ -2452,19 +2452,19 @@ int workspace_ensure(Workspace *ws, const DevGraph &g, int nqueries, cudaStream_
     if (ws->ctl && ws->V == g.V) {
         if (nqueries <= ws->ctl_cap) return TRAV_OK;
         TRY_CUDA(cudaStreamSynchronize(st));
-        dev_free(ws->ctl);
+        dev_free(ws->ctl, st);
         ws->ctl = nullptr;
         ws->ctl_cap = 0;
         TRY_CUDA(dev_malloc(&ws->ctl, sizeof(Ctl) * (size_t)nqueries));
         ws->ctl_cap = nqueries;
         return TRAV_OK;
     }
-    workspace_free(ws);
+    workspace_free(ws, st);
     const int64_t V = g.V > 0 ? g.V : 1;
     const int64_t W = (V + 31) / 32;
     ws->V = g.V;
     ws->chunk_cap = V + g.E / kMinItem + 1;
-    DevSlab mem;
+    DevSlab mem(st);
     unsigned long long *words = nullptr;
     mem.add(&words, V);
     mem.add(&ws->rcls, V);
@@ -2485,13 +2485,13 @@ int workspace_ensure(Workspace *ws, const DevGraph &g, int nqueries, cudaStream_
     return TRAV_OK;
 }
 
-void workspace_free(Workspace *ws)
+void workspace_free(Workspace *ws, cudaStream_t st)
 {
-    dev_free(ws->mem);
-    light_rows_free(&ws->light);
-    dev_free(ws->ctl);
-    dev_free(ws->plan[0]);
-    dev_free(ws->plan[1]);
+    dev_free(ws->mem, st);
+    light_rows_free(&ws->light, st);
+    dev_free(ws->ctl, st);
+    dev_free(ws->plan[0], nullptr);  // written on the legacy stream
+    dev_free(ws->plan[1], nullptr);
     *ws = Workspace{};
 }
 
@@ -2636,7 +2636,7 @@ int query_bytes(const DevGraph &g, Workspace *ws, int q, int kind, int64_t *byte
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, acc, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    dev_free(acc);
+    dev_free(acc, st);
     if (e != cudaSuccess) return cuda_fail(e, "query_bytes");
     *reached = (int64_t)h[0];
     *reached_edges = (int64_t)h[1];

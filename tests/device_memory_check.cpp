@@ -1,0 +1,157 @@
+// The library's device-memory management (csrc/device_memory.cu) on a CUDA runtime of the host: one scenario a run.
+#include "fake_cudart.hpp"
+
+#include "../parallel-task1_b200/csrc/device_memory.cu"
+
+#include <cstdio>
+#include <cstring>
+#include <random>
+#include <thread>
+
+using namespace trav;
+
+static int g_bad = 0;
+#define CHECK(x)                                                      \
+    do {                                                              \
+        if (!(x)) {                                                   \
+            std::printf("line %d: not so: %s\n", __LINE__, #x);       \
+            g_bad = 1;                                                \
+        }                                                             \
+    } while (0)
+
+static const size_t MB = size_t(1) << 20;
+
+static void *get(size_t bytes)
+{
+    void *p = nullptr;
+    CHECK(dev_malloc_bytes(&p, bytes) == cudaSuccess && p);
+    return p;
+}
+static cudaStream_t stream()
+{
+    cudaStream_t st = nullptr;
+    CHECK(stream_get(&st) == cudaSuccess && st);
+    return st;
+}
+
+// A freed block goes to the next owner of about its size, once the stream of its last work has been waited for.
+static void reuse()
+{
+    cudaStream_t a = stream();
+    void *p = get(10 * MB);
+    fake::streams[a].busy = true;
+    dev_free(p, a);
+    CHECK(!fake::streams[a].busy);
+    CHECK(get(20 * MB) != p);
+    CHECK(get(10 * MB - 100) == p);  // on whatever stream
+    CHECK(get(10 * MB) != p);
+    CHECK(fake::count("free") == 0);
+}
+
+// Another stream is being captured: no wait for the device, no error left behind, and the block is kept.
+static void capture()
+{
+    cudaStream_t a = stream(), b = stream();
+    fake::streams[b].captured = true;
+    void *p = get(10 * MB);
+    dev_free(p, a);
+    CHECK(cudaGetLastError() == cudaSuccess);
+    CHECK(fake::count("device wait") == 0);
+    CHECK(get(10 * MB) == p);
+    // a wait that fails leaves no error for the caller's next launch, and the block is not kept
+    dev_free(p, b);
+    CHECK(cudaGetLastError() == cudaSuccess);
+    CHECK(fake::count("free") == 1);
+}
+
+// What is kept stays below the bound: the oldest blocks go, and a block above the bound is not kept at all.
+static void bound()
+{
+    cudaStream_t a = stream();
+    void *big = get(1025 * MB);
+    dev_free(big, a);
+    CHECK(fake::used == 0);
+    std::vector<void *> p;
+    for (int i = 0; i < 12; i++) p.push_back(get(100 * MB));
+    for (void *x : p) {
+        dev_free(x, a);
+    }
+    CHECK(fake::used == 1000 * MB);
+    CHECK(!fake::allocs.count(p[0]) && !fake::allocs.count(p[1]) && fake::allocs.count(p[2]));
+}
+
+// An allocation that does not fit beside the kept blocks gets their memory; one that cannot fit fails.
+static void give_back()
+{
+    cudaStream_t a = stream();
+    fake::capacity = 1000 * MB;
+    void *p = get(600 * MB);
+    dev_free(p, a);
+    void *q = get(900 * MB);
+    CHECK(fake::used == 900 * MB);
+    void *r = nullptr;
+    CHECK(dev_malloc_bytes(&r, 200 * MB) == cudaErrorMemoryAllocation && !r);
+    dev_free(q, a);
+    CHECK(get(1000 * MB) != nullptr);
+    arm_alloc_failure(0);
+    CHECK(dev_malloc_bytes(&r, 1) == cudaErrorMemoryAllocation && !r);
+}
+
+// Several threads: no block has two owners.
+static void threads()
+{
+    std::mutex mu;
+    std::map<void *, int> owner;
+    std::vector<std::thread> ts;
+    for (int t = 0; t < 8; t++)
+        ts.emplace_back([&, t] {
+            std::mt19937 rng(t);
+            cudaStream_t st = nullptr;
+            CHECK(stream_get(&st) == cudaSuccess);
+            std::vector<void *> mine;
+            for (int k = 0; k < 4000; k++) {
+                if (mine.empty() || rng() % 2) {
+                    void *p = nullptr;
+                    CHECK(dev_malloc_bytes(&p, (1 + rng() % 40) * MB) == cudaSuccess);
+                    std::lock_guard<std::mutex> lock(mu);
+                    CHECK(owner.emplace(p, t).second);
+                    mine.push_back(p);
+                } else {
+                    std::swap(mine[rng() % mine.size()], mine.back());
+                    {
+                        std::lock_guard<std::mutex> lock(mu);
+                        CHECK(owner[mine.back()] == t);
+                        owner.erase(mine.back());
+                    }
+                    dev_free(mine.back(), st);
+                    mine.pop_back();
+                }
+            }
+            for (void *p : mine) {
+                {
+                    std::lock_guard<std::mutex> lock(mu);
+                    owner.erase(p);
+                }
+                dev_free(p, st);
+            }
+            stream_put(st);
+        });
+    for (auto &t : ts) t.join();
+    CHECK(fake::used <= 1024 * MB);
+    CHECK(fake::count("waited for a stream that is gone") == 0);
+}
+
+int main(int argc, char **argv)
+{
+    const struct {
+        const char *name;
+        void (*run)();
+    } all[] = {{"reuse", reuse}, {"capture", capture}, {"bound", bound}, {"give_back", give_back}, {"threads", threads}};
+    for (const auto &s : all)
+        if (argc == 2 && !std::strcmp(argv[1], s.name)) {
+            s.run();
+            return g_bad;
+        }
+    std::printf("unknown scenario\n");
+    return 2;
+}

@@ -1,0 +1,139 @@
+// A CUDA runtime of the host for tests of the library's memory management: allocations, streams, captures and
+// contexts are records that the test looks at, and calls follow the documented rules (a device-wide wait is
+// refused while any stream is captured, memory of an ended context is gone, and so on).  Compiled into the test
+// program together with csrc/device_memory.cu; no device is needed.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <map>
+#include <mutex>
+#include <string>
+#include <vector>
+
+static const uint3 blockIdx{}, threadIdx{};
+
+namespace fake {
+
+struct Alloc {
+    size_t bytes;
+    unsigned long long id;
+    int context;
+};
+struct Stream {
+    bool busy = false;
+    bool captured = false;
+    int context = 0;
+};
+
+inline std::mutex mu;
+inline std::map<void *, Alloc> allocs;
+inline std::map<cudaStream_t, Stream> streams;  // key 0: the legacy stream
+inline std::vector<std::string> log;
+inline size_t capacity = size_t(180) << 30, used = 0;
+inline unsigned long long next_id = 1;
+inline unsigned char *next_at = reinterpret_cast<unsigned char *>(0x700000000000ull);
+inline int context = 1;  // the context that lives now
+inline cudaError_t last = cudaSuccess;
+
+inline cudaError_t fail(cudaError_t e) { return last = e; }
+inline size_t count(const std::string &what)
+{
+    size_t n = 0;
+    for (const std::string &s : log) n += s == what;
+    return n;
+}
+// What cudaDeviceReset leaves: no allocation, no stream, another context at the next call.
+inline void reset()
+{
+    allocs.clear();
+    streams.clear();
+    used = 0;
+    context++;
+}
+
+}  // namespace fake
+
+extern "C" {
+
+cudaError_t cudaMalloc(void **p, size_t bytes)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    using namespace fake;
+    log.push_back("malloc");
+    if (used + bytes > capacity) return fail(cudaErrorMemoryAllocation);
+    *p = next_at;
+    next_at += (bytes + 511) & ~size_t(511);
+    allocs[*p] = Alloc{bytes, next_id++, context};
+    used += bytes;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    using namespace fake;
+    if (!p) return cudaSuccess;
+    log.push_back("free");
+    auto it = allocs.find(p);
+    if (it == allocs.end()) return fail(cudaErrorInvalidValue);
+    used -= it->second.bytes;
+    allocs.erase(it);
+    return cudaSuccess;
+}
+cudaError_t cudaMemGetInfo(size_t *f, size_t *t)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    *f = fake::capacity - fake::used;
+    *t = fake::capacity;
+    return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    const cudaError_t e = fake::last;
+    fake::last = cudaSuccess;
+    return e;
+}
+cudaError_t cudaDeviceSynchronize()
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    using namespace fake;
+    log.push_back("device wait");
+    for (auto &s : streams)
+        if (s.second.captured) return fail(cudaErrorStreamCaptureUnsupported);
+    for (auto &s : streams) s.second.busy = false;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *st, unsigned)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    using namespace fake;
+    static unsigned long long at = 0x1000;
+    log.push_back("stream create");
+    *st = reinterpret_cast<cudaStream_t>(at += 16);
+    streams[*st] = Stream{false, false, context};
+    return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t st)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    using namespace fake;
+    log.push_back("stream destroy");
+    if (!streams.erase(st)) log.push_back("destroyed a stream that is gone");
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t st)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    using namespace fake;
+    if (st && !streams.count(st)) {
+        log.push_back("waited for a stream that is gone");
+        return fail(cudaErrorInvalidResourceHandle);
+    }
+    if (streams[st].captured) return fail(cudaErrorStreamCaptureUnsupported);
+    streams[st].busy = false;
+    return cudaSuccess;
+}
+
+}  // extern "C"
