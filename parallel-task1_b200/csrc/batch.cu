@@ -282,11 +282,12 @@ int run_launch(trav_batch *b, int32_t n, const trav_batch_shape &s, float *ms, u
     if (teams > b->teams_alloc) {
         // every team needs scratch for the batch's largest graph: run fewer
         // teams (each still of team_ctas CTAs) when the device cannot hold them
-        size_t free_b = 0, total_b = 0;
-        TRY_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        const size_t have = (size_t)b->teams_alloc * b->team_bytes + free_b;
         const size_t spare = (size_t)1 << 30;  // left for the caller
         const size_t per = team_layout(b).total + sizeof(Ctl) + sizeof(TeamWs);
+        const size_t held = (size_t)b->teams_alloc * b->team_bytes;
+        size_t free_b = 0;
+        TRY_CUDA(dev_free_bytes(spare + per * (size_t)teams - held, &free_b));
+        const size_t have = held + free_b;
         const size_t fit = have > spare ? (have - spare) / per : 0;
         if (fit < 1) {
             set_error("batch: not enough device memory for one team's scratch");

@@ -229,7 +229,11 @@ int run_batch(trav_graph *g, int kind, const int32_t *sources, int32_t n, const 
                 return rc;
             }
             if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
-            const cudaError_t ei = cudaGraphInstantiate(&c.exec, graph, 0);
+            cudaError_t ei = cudaGraphInstantiate(&c.exec, graph, 0);
+            if (ei == cudaErrorMemoryAllocation && dev_trim() > 0) {
+                cudaGetLastError();
+                ei = cudaGraphInstantiate(&c.exec, graph, 0);
+            }
             cudaGraphDestroy(graph);
             if (ei != cudaSuccess) return cuda_fail(ei, "cudaGraphInstantiate");
             c.key = std::move(key);

@@ -106,15 +106,8 @@ cudaError_t dev_malloc_bytes(void **p, size_t bytes)
         }
     }
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        std::vector<void *> out;
-        {
-            std::lock_guard<std::mutex> lock(g_mu);
-            out = take_over(dev, 0);
-        }
-        if (out.empty()) return e;
+    if (e == cudaErrorMemoryAllocation && dev_trim() > 0) {
         cudaGetLastError();
-        for (void *q : out) cudaFree(q);
         e = cudaMalloc(p, bytes);
     }
     if (e != cudaSuccess) {
@@ -124,6 +117,28 @@ cudaError_t dev_malloc_bytes(void **p, size_t bytes)
     std::lock_guard<std::mutex> lock(g_mu);
     g_live[*p] = Block{*p, bytes, dev};
     return cudaSuccess;
+}
+
+size_t dev_trim()
+{
+    const int dev = current_device();
+    size_t bytes = 0;
+    std::vector<void *> out;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        for (const Block &b : g_kept) bytes += b.device == dev ? b.bytes : 0;
+        out = take_over(dev, 0);
+    }
+    for (void *q : out) cudaFree(q);
+    return bytes;
+}
+
+cudaError_t dev_free_bytes(size_t want, size_t *bytes)
+{
+    size_t total = 0;
+    cudaError_t e = cudaMemGetInfo(bytes, &total);
+    if (e == cudaSuccess && *bytes < want && dev_trim() > 0) e = cudaMemGetInfo(bytes, &total);
+    return e;
 }
 
 void dev_free(void *p, cudaStream_t st)

@@ -284,6 +284,11 @@ bool is_device_ptr(const void *p);
 // allocation fails with cudaErrorMemoryAllocation as cudaMalloc would.
 cudaError_t dev_malloc_bytes(void **p, size_t bytes);
 void dev_free(void *p, cudaStream_t st);
+// Give the kept blocks of the current device back; returns their bytes.
+size_t dev_trim();
+// Free bytes of the current device.  Kept blocks are given back first when that
+// is less than `want`: for callers that decide by it what they ask for.
+cudaError_t dev_free_bytes(size_t want, size_t *bytes);
 // True when the armed failure falls on this allocation (each array of a DevSlab counts as one).
 bool alloc_failure_due();
 void arm_alloc_failure(int32_t after);

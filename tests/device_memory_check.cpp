@@ -97,6 +97,21 @@ static void give_back()
     CHECK(dev_malloc_bytes(&r, 1) == cudaErrorMemoryAllocation && !r);
 }
 
+// What is kept counts as free where the free memory decides what is asked for.
+static void counts_as_free()
+{
+    cudaStream_t a = stream();
+    fake::capacity = 1000 * MB;
+    get(300 * MB);
+    dev_free(get(200 * MB), a);
+    size_t bytes = 0;
+    CHECK(dev_free_bytes(400 * MB, &bytes) == cudaSuccess && bytes == 500 * MB);
+    CHECK(fake::count("free") == 0);  // enough: the block stays
+    CHECK(dev_free_bytes(600 * MB, &bytes) == cudaSuccess && bytes == 700 * MB);
+    CHECK(fake::count("free") == 1 && dev_trim() == 0);
+    CHECK(dev_free_bytes(900 * MB, &bytes) == cudaSuccess && bytes == 700 * MB);
+}
+
 // Several threads: no block has two owners.
 static void threads()
 {
@@ -146,7 +161,8 @@ int main(int argc, char **argv)
     const struct {
         const char *name;
         void (*run)();
-    } all[] = {{"reuse", reuse}, {"capture", capture}, {"bound", bound}, {"give_back", give_back}, {"threads", threads}};
+    } all[] = {{"reuse", reuse}, {"capture", capture}, {"bound", bound}, {"give_back", give_back},
+                {"counts_as_free", counts_as_free}, {"threads", threads}};
     for (const auto &s : all)
         if (argc == 2 && !std::strcmp(argv[1], s.name)) {
             s.run();

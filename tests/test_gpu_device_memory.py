@@ -45,3 +45,30 @@ def test_graphs_built_and_freed_in_one_thread_do_not_disturb_a_capture_in_anothe
     assert not errors, errors
     assert np.array_equal(out.cpu().numpy(), np.stack(want))
     g.free()
+
+
+def test_a_batch_runs_in_the_memory_that_the_library_keeps():
+    """Little is free beside kept blocks: the teams' scratch is sized as if they were free, as they were before
+    blocks were kept."""
+    import torch
+
+    V = 1 << 10
+    s, d, w = O.rmat(10, 8, seed=3)
+    src, dst, _ = O.rmat(19, 16, seed=4)
+    b = T.Batch([g := T.Graph.from_edges(V, s, d, w)])
+    levels = torch.empty((8, V), dtype=torch.int32, device="cuda")
+    queries = [(0, 0, x, 0.0, T.SCHEDULE_PLAIN, levels[x]) for x in range(8)]
+    T.Graph.from_edges(1 << 19, src, dst, None).free()  # leaves some 600 MB of kept blocks
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    # less than the 1 GB that a batch leaves to the caller, more with the kept blocks
+    filler = torch.empty(free - (900 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 1 << 30
+        b.run(queries)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert np.array_equal(levels.cpu().numpy(), np.stack([O.bfs_levels(V, s, d, x) for x in range(8)]))
+    b.close()
+    g.free()
