@@ -361,6 +361,15 @@ int trav_last_decisions(trav_graph *g, float *x, uint8_t *choice, int32_t *phase
 
 /* ------------------------------------------------------------------- misc */
 
+/* Give the device memory that the library keeps on the current device back to
+ * the driver.  Freed handles, batches and scratch leave their blocks for the
+ * next allocation of about their size, up to 1 GB a device (what no handle or
+ * batch uses: those in use stay as they are).  The library gives them back by
+ * itself when an allocation of its own needs them; call this before another
+ * allocator in the process does.  *bytes (may be NULL) receives how much it
+ * was.  No counterpart in the reference. */
+int trav_trim_memory(int64_t *bytes);
+
 const char *trav_last_error(void);
 const char *trav_version(void);
 

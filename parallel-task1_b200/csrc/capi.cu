@@ -277,6 +277,14 @@ const char *trav_last_error(void) { return g_err.c_str(); }
 
 const char *trav_version(void) { return "trav-b200 0.1 (sm_100a)"; }
 
+int trav_trim_memory(int64_t *bytes)
+{
+    TRY(check_device());
+    const size_t n = dev_trim();
+    if (bytes) *bytes = (int64_t)n;
+    return TRAV_OK;
+}
+
 int trav_inject_alloc_failure(int32_t after)
 {
     if (after < -1) return bad("after must be >= -1");

@@ -54,7 +54,7 @@ EXPORTS = [
     "trav_el_optimize", "trav_el_gpu_transactions", "trav_adj_file_read", "trav_adj_file_write",
     "trav_pairs_file_read", "trav_set_limits", "trav_inject_alloc_failure", "trav_reach_el_masked",
     "trav_mlp_set_margin", "trav_batch_run_host", "trav_tune_table_save", "trav_tune_table_load",
-    "trav_set_sssp_split", "trav_graph_mean_weight",
+    "trav_set_sssp_split", "trav_graph_mean_weight", "trav_trim_memory",
 ]
 
 
@@ -150,6 +150,7 @@ def lib():
         L.trav_set_plan.argtypes = [vp, i32, vp, i32]
         L.trav_set_limits.argtypes = [vp, i32, C.c_uint64]
         L.trav_inject_alloc_failure.argtypes = [i32]
+        L.trav_trim_memory.argtypes = [C.POINTER(i64)]
         L.trav_last_decisions.argtypes = [vp, vp, vp, vp, vp, vp, i32, C.POINTER(i32)]
         _lib = L
     return _lib
@@ -432,6 +433,14 @@ def bellman_ford_wrapper(src, dst, w, V: int, E: int, source: int, d):
 def bfs_wrapper(src, dst, V: int, E: int, visited, source: int):
     """bfs_wrapper on CUDA tensors; visited is a uint8/bool CUDA tensor of V entries."""
     _check(lib().trav_bfs_el(_ptr(src), _ptr(dst), V, E, _ptr(visited), source))
+
+
+def trim_memory() -> int:
+    """Give the device memory that the library keeps for its next allocations (at most 1 GB) back to the driver, for
+    other allocators of the process; returns the bytes."""
+    n = C.c_int64(0)
+    _check(lib().trav_trim_memory(C.byref(n)))
+    return n.value
 
 
 def inject_alloc_failure(after: int):

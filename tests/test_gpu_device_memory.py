@@ -72,3 +72,25 @@ def test_a_batch_runs_in_the_memory_that_the_library_keeps():
     assert np.array_equal(levels.cpu().numpy(), np.stack([O.bfs_levels(V, s, d, x) for x in range(8)]))
     b.close()
     g.free()
+
+
+def test_kept_memory_is_bounded_and_given_back_on_request():
+    import torch
+
+    V = 1 << 18
+    s, d, w = O.rmat(18, 16, seed=9)
+    hub = int(np.bincount(s, minlength=V).argmax())
+    want = O.bfs_levels(V, s, d, hub)
+    T.trim_memory()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(12):
+        graphs = [T.Graph.from_edges(V, s, d, w) for _ in range(4)]
+        assert np.array_equal(graphs[-1].bfs([hub])[0], want)  # in blocks of earlier handles
+        for g in graphs:
+            g.free()
+    kept = free - torch.cuda.mem_get_info()[0]
+    assert 0 < kept <= (1 << 30) + (64 << 20)  # the driver hands out pages of 2 MB
+    assert T.trim_memory() > 0
+    assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
+    assert T.trim_memory() == 0
