@@ -81,6 +81,9 @@ def test_kept_memory_is_bounded_and_given_back_on_request():
     s, d, w = O.rmat(18, 16, seed=9)
     hub = int(np.bincount(s, minlength=V).argmax())
     want = O.bfs_levels(V, s, d, hub)
+    g = T.Graph.from_edges(V, s, d, w)
+    g.bfs([hub])  # what a first call loads is there
+    g.free()
     T.trim_memory()
     torch.cuda.synchronize()
     free = torch.cuda.mem_get_info()[0]
