@@ -16,6 +16,12 @@
 // work), so its next owner may use it on any stream.  A wait for the whole device
 // would do the same, but CUDA refuses one while any of its streams is captured,
 // and the capture, another thread's perhaps, is lost.
+//
+// Blocks and streams belong to the context they were made in, and are gone when
+// it ends (cudaDeviceReset).  So they are kept by context, and each context's
+// keeps hold a mark: an allocation whose buffer id, which no other allocation of
+// the process ever has, is asked for before anything is handed out.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -31,18 +37,32 @@ namespace {
 
 constexpr size_t kKeepBytes = size_t(1024) << 20;
 constexpr size_t kKeepStreams = 8;
+constexpr size_t kMarkBytes = 512;
 
 struct Block {
     void *p;
     size_t bytes;
     int device;
+    unsigned long long epoch;  // of its context (0: unknown)
+};
+
+// What is kept of one context.
+struct Context {
+    CUcontext handle;
+    unsigned long long epoch;  // no other context of the process has it, a later one at the same address neither
+    void *mark;
+    unsigned long long mark_id;
+    std::list<Block> kept;     // idle blocks, oldest first
+    std::vector<cudaStream_t> streams;  // idle streams
 };
 
 // never destroyed: handles may be freed while the process exits
 std::mutex &g_mu = *new std::mutex;
 std::unordered_map<void *, Block> &g_live = *new std::unordered_map<void *, Block>;  // blocks handed out
-std::list<Block> &g_kept = *new std::list<Block>;                                    // idle blocks, oldest first
-std::vector<std::pair<int, cudaStream_t>> &g_streams = *new std::vector<std::pair<int, cudaStream_t>>;  // idle streams
+std::unordered_map<cudaStream_t, unsigned long long> &g_live_streams =
+    *new std::unordered_map<cudaStream_t, unsigned long long>;  // streams handed out, and their contexts' epochs
+std::list<Context> &g_contexts = *new std::list<Context>;
+unsigned long long g_epochs = 0;
 
 // Allocations left before the injected failure (-1: none armed).
 std::atomic<int64_t> g_fail_after{-1};
@@ -54,20 +74,96 @@ int current_device()
     return d;
 }
 
-// Take idle blocks of `device` out of the list, oldest first, until those left hold at most `keep` bytes.
-std::vector<void *> take_over(int device, size_t keep)
+// The two driver calls that know about contexts (the runtime has none, and the
+// library does not link the driver, which a machine without a GPU lacks).
+struct Driver {
+    CUresult (*current)(CUcontext *) = nullptr;
+    CUresult (*attribute)(void *, CUpointer_attribute, CUdeviceptr) = nullptr;
+    Driver()
+    {
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", (void **)&current, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", (void **)&attribute, 12000, cudaEnableDefault, &r) != cudaSuccess) {
+            cudaGetLastError();
+            current = nullptr;
+        }
+    }
+    CUcontext context() const
+    {
+        CUcontext c = nullptr;
+        return current(&c) == CUDA_SUCCESS ? c : nullptr;
+    }
+    unsigned long long buffer_id(void *p) const  // 0: no allocation
+    {
+        unsigned long long id = 0;
+        return attribute(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, (CUdeviceptr)p) == CUDA_SUCCESS ? id : 0;
+    }
+};
+
+const Driver &the_driver()
+{
+    static const Driver d;
+    return d;
+}
+
+// The keeps of the current context (g_mu held); nullptr: nothing can be kept.
+Context *context_here()
+{
+    const Driver &driver = the_driver();
+    if (!driver.current || !driver.attribute) return nullptr;
+    CUcontext c = driver.context();
+    if (!c) {
+        // a thread's first call: the runtime makes the device's context current
+        if (cudaFree(nullptr) != cudaSuccess) cudaGetLastError();
+        c = driver.context();
+    }
+    for (auto it = g_contexts.begin(); c && it != g_contexts.end(); ++it) {
+        if (it->handle != c) continue;
+        if (driver.buffer_id(it->mark) == it->mark_id) return &*it;
+        // that context has ended, and its blocks and streams with it
+        g_contexts.erase(it);
+        break;
+    }
+    Context n{nullptr, 0, nullptr, 0, {}, {}};
+    if (cudaMalloc(&n.mark, kMarkBytes) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    n.handle = driver.context();
+    n.mark_id = driver.buffer_id(n.mark);
+    if (!n.handle || !n.mark_id) {
+        cudaFree(n.mark);
+        return nullptr;
+    }
+    n.epoch = ++g_epochs;
+    n.streams.reserve(kKeepStreams);
+    g_contexts.push_back(n);
+    return &g_contexts.back();
+}
+
+// Whether the context of this epoch is not known to have ended (g_mu held).
+bool lives(unsigned long long epoch)
+{
+    if (epoch == 0) return true;
+    for (auto it = g_contexts.begin(); it != g_contexts.end(); ++it) {
+        if (it->epoch != epoch) continue;
+        if (the_driver().buffer_id(it->mark) == it->mark_id) return true;
+        g_contexts.erase(it);
+        break;
+    }
+    return false;
+}
+
+// Take idle blocks of a context out of its list, oldest first, until those left hold at most `keep` bytes.
+std::vector<void *> take_over(Context *c, size_t keep)
 {
     size_t held = 0;
-    for (const Block &b : g_kept) held += b.device == device ? b.bytes : 0;
+    for (const Block &b : c->kept) held += b.bytes;
     std::vector<void *> out;
-    for (auto it = g_kept.begin(); it != g_kept.end() && held > keep;) {
-        if (it->device != device) {
-            ++it;
-            continue;
-        }
-        held -= it->bytes;
-        out.push_back(it->p);
-        it = g_kept.erase(it);
+    while (!c->kept.empty() && held > keep) {
+        held -= c->kept.front().bytes;
+        out.push_back(c->kept.front().p);
+        c->kept.pop_front();
     }
     return out;
 }
@@ -84,25 +180,35 @@ bool alloc_failure_due()
     return false;
 }
 
+unsigned long long context_epoch()
+{
+    std::lock_guard<std::mutex> lock(g_mu);
+    const Context *c = context_here();
+    return c ? c->epoch : 0;
+}
+
 cudaError_t dev_malloc_bytes(void **p, size_t bytes)
 {
     *p = nullptr;
     if (alloc_failure_due()) return cudaErrorMemoryAllocation;
-    const int dev = current_device();
     bytes = (bytes + 511) & ~(size_t)511;
     if (bytes == 0) bytes = 512;
+    unsigned long long epoch = 0;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        auto best = g_kept.end();
-        for (auto it = g_kept.begin(); it != g_kept.end(); ++it)
-            if (it->device == dev && it->bytes >= bytes && it->bytes <= bytes + bytes / 4 + 4096 &&
-                (best == g_kept.end() || it->bytes < best->bytes))
-                best = it;
-        if (best != g_kept.end()) {
-            *p = best->p;
-            g_live[best->p] = *best;
-            g_kept.erase(best);
-            return cudaSuccess;
+        if (Context *c = context_here()) {
+            epoch = c->epoch;
+            auto best = c->kept.end();
+            for (auto it = c->kept.begin(); it != c->kept.end(); ++it)
+                if (it->bytes >= bytes && it->bytes <= bytes + bytes / 4 + 4096 &&
+                    (best == c->kept.end() || it->bytes < best->bytes))
+                    best = it;
+            if (best != c->kept.end()) {
+                *p = best->p;
+                g_live[best->p] = *best;
+                c->kept.erase(best);
+                return cudaSuccess;
+            }
         }
     }
     cudaError_t e = cudaMalloc(p, bytes);
@@ -115,19 +221,20 @@ cudaError_t dev_malloc_bytes(void **p, size_t bytes)
         return e;
     }
     std::lock_guard<std::mutex> lock(g_mu);
-    g_live[*p] = Block{*p, bytes, dev};
+    g_live[*p] = Block{*p, bytes, current_device(), epoch};
     return cudaSuccess;
 }
 
 size_t dev_trim()
 {
-    const int dev = current_device();
     size_t bytes = 0;
     std::vector<void *> out;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        for (const Block &b : g_kept) bytes += b.device == dev ? b.bytes : 0;
-        out = take_over(dev, 0);
+        if (Context *c = context_here()) {
+            for (const Block &b : c->kept) bytes += b.bytes;
+            out = take_over(c, 0);
+        }
     }
     for (void *q : out) cudaFree(q);
     return bytes;
@@ -144,7 +251,7 @@ cudaError_t dev_free_bytes(size_t want, size_t *bytes)
 void dev_free(void *p, cudaStream_t st)
 {
     if (!p) return;
-    Block b{p, 0, -1};
+    Block b{p, 0, -1, 0};
     {
         std::lock_guard<std::mutex> lock(g_mu);
         auto it = g_live.find(p);
@@ -153,51 +260,64 @@ void dev_free(void *p, cudaStream_t st)
             g_live.erase(it);
         }
     }
-    if (b.device < 0 || b.bytes > kKeepBytes) {
+    if (b.device < 0) {
         cudaFree(p);
         return;
     }
-    // nothing may still read or write the block when it is handed on
     const int cur = current_device();
     if (cur != b.device) cudaSetDevice(b.device);
+    // nothing may still read or write the block when it is handed on
     const cudaError_t e = cudaStreamSynchronize(st);
-    if (cur != b.device) cudaSetDevice(cur);
-    if (e != cudaSuccess) {
-        cudaGetLastError();  // not the caller's next launch's
-        cudaFree(p);
-        return;
-    }
+    if (e != cudaSuccess) cudaGetLastError();  // not the caller's next launch's
     std::vector<void *> out;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        out = take_over(b.device, kKeepBytes - b.bytes);
-        g_kept.push_back(b);
+        Context *c = context_here();
+        if (e == cudaSuccess && c && c->epoch == b.epoch && b.bytes <= kKeepBytes) {
+            out = take_over(c, kKeepBytes - b.bytes);
+            c->kept.push_back(b);
+        } else if (lives(b.epoch)) {
+            out.push_back(p);
+        }
     }
     for (void *q : out) cudaFree(q);
+    if (cur != b.device) cudaSetDevice(cur);
 }
 
 cudaError_t stream_get(cudaStream_t *st)
 {
-    const int dev = current_device();
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        for (auto it = g_streams.begin(); it != g_streams.end(); ++it)
-            if (it->first == dev) {
-                *st = it->second;
-                g_streams.erase(it);
-                return cudaSuccess;
-            }
+    std::lock_guard<std::mutex> lock(g_mu);
+    Context *c = context_here();
+    if (c && !c->streams.empty()) {
+        *st = c->streams.back();
+        c->streams.pop_back();
+    } else {
+        const cudaError_t e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+        if (e != cudaSuccess) return e;
     }
-    return cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+    g_live_streams[*st] = c ? c->epoch : 0;
+    return cudaSuccess;
 }
 
 void stream_put(cudaStream_t st)
 {
     if (!st) return;
+    unsigned long long epoch = 0;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto it = g_live_streams.find(st);
+        if (it != g_live_streams.end()) {
+            epoch = it->second;
+            g_live_streams.erase(it);
+        }
+        context_here();
+        if (!lives(epoch)) return;
+    }
     if (cudaStreamSynchronize(st) == cudaSuccess) {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (g_streams.size() < kKeepStreams) {
-            g_streams.emplace_back(current_device(), st);
+        Context *c = context_here();
+        if (c && c->epoch == epoch && c->streams.size() < kKeepStreams) {
+            c->streams.push_back(st);
             return;
         }
     }

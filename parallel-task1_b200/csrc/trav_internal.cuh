@@ -289,6 +289,9 @@ size_t dev_trim();
 // Free bytes of the current device.  Kept blocks are given back first when that
 // is less than `want`: for callers that decide by it what they ask for.
 cudaError_t dev_free_bytes(size_t want, size_t *bytes);
+// A number that the current context shares with no other of the process, not
+// even with one that follows it (0: not known).  For what is set up once a context.
+unsigned long long context_epoch();
 // True when the armed failure falls on this allocation (each array of a DevSlab counts as one).
 bool alloc_failure_due();
 void arm_alloc_failure(int32_t after);

@@ -2222,11 +2222,12 @@ constexpr int64_t kNarrowAloneEdges = 1 << 18;
 int narrow_ctas(int kind)
 {
     constexpr int kMaxDevices = 64;
-    static std::atomic<int> known[2][kMaxDevices];  // CTAs + 1
+    // context << 8 | CTAs: the kernel's attributes, set below, are the context's
+    static std::atomic<unsigned long long> known[2][kMaxDevices];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    const int k = known[kind][dev].load();
-    if (k) return k - 1;
+    const unsigned long long epoch = context_epoch(), k = known[kind][dev].load();
+    if (epoch && k >> 8 == epoch) return (int)(k & 255u);
     const void *fn = kind == 0 ? (const void *)bfs_narrow : (const void *)sssp_narrow;
     int found = 0;
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(NarrowShared)) == cudaSuccess &&
@@ -2247,7 +2248,7 @@ int narrow_ctas(int kind)
         }
     }
     cudaGetLastError();
-    known[kind][dev].store(found + 1);
+    if (epoch) known[kind][dev].store(epoch << 8 | (unsigned)found);
     return found;
 }
 

@@ -3,7 +3,10 @@
 // refused while any stream is captured, memory of an ended context is gone, and so on).  Compiled into the test
 // program together with csrc/device_memory.cu; no device is needed.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
+
+#include <cstring>
 
 #include <map>
 #include <mutex>
@@ -31,8 +34,11 @@ inline std::map<cudaStream_t, Stream> streams;  // key 0: the legacy stream
 inline std::vector<std::string> log;
 inline size_t capacity = size_t(180) << 30, used = 0;
 inline unsigned long long next_id = 1;
-inline unsigned char *next_at = reinterpret_cast<unsigned char *>(0x700000000000ull);
-inline int context = 1;  // the context that lives now
+inline unsigned char *const first_at = reinterpret_cast<unsigned char *>(0x700000000000ull), *next_at = first_at;
+inline int context = 1;       // the context that lives now
+inline bool current = false;  // and whether it is current yet (in any thread: there is one)
+inline CUcontext handle = reinterpret_cast<CUcontext>(0x10);  // where the driver keeps it
+inline bool driver = true;    // the driver's entry points can be found
 inline cudaError_t last = cudaSuccess;
 
 inline cudaError_t fail(cudaError_t e) { return last = e; }
@@ -42,9 +48,13 @@ inline size_t count(const std::string &what)
     for (const std::string &s : log) n += s == what;
     return n;
 }
-// What cudaDeviceReset leaves: no allocation, no stream, another context at the next call.
-inline void reset()
+// What cudaDeviceReset leaves: no allocation, no stream, and another context at the next call, which the driver may
+// keep where the old one was and whose memory may begin where the old one's did.
+inline void reset(CUcontext at, bool same_addresses)
 {
+    handle = at;
+    if (same_addresses) next_at = first_at;
+    current = false;
     allocs.clear();
     streams.clear();
     used = 0;
@@ -60,6 +70,7 @@ cudaError_t cudaMalloc(void **p, size_t bytes)
     std::lock_guard<std::mutex> lock(fake::mu);
     using namespace fake;
     log.push_back("malloc");
+    current = true;
     if (used + bytes > capacity) return fail(cudaErrorMemoryAllocation);
     *p = next_at;
     next_at += (bytes + 511) & ~size_t(511);
@@ -71,6 +82,7 @@ cudaError_t cudaFree(void *p)
 {
     std::lock_guard<std::mutex> lock(fake::mu);
     using namespace fake;
+    current = true;
     if (!p) return cudaSuccess;
     log.push_back("free");
     auto it = allocs.find(p);
@@ -133,6 +145,31 @@ cudaError_t cudaStreamSynchronize(cudaStream_t st)
     }
     if (streams[st].captured) return fail(cudaErrorStreamCaptureUnsupported);
     streams[st].busy = false;
+    return cudaSuccess;
+}
+
+CUresult fake_cuCtxGetCurrent(CUcontext *c)
+{
+    *c = fake::current ? fake::handle : nullptr;
+    return CUDA_SUCCESS;
+}
+CUresult fake_cuPointerGetAttribute(void *out, CUpointer_attribute what, CUdeviceptr p)
+{
+    std::lock_guard<std::mutex> lock(fake::mu);
+    auto it = fake::allocs.find(reinterpret_cast<void *>(p));
+    if (what != CU_POINTER_ATTRIBUTE_BUFFER_ID || it == fake::allocs.end()) return CUDA_ERROR_INVALID_VALUE;
+    *static_cast<unsigned long long *>(out) = it->second.id;
+    return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char *name, void **fn, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult *r)
+{
+    *fn = nullptr;
+    *r = cudaDriverEntryPointSymbolNotFound;
+    if (!fake::driver) return fake::fail(cudaErrorInsufficientDriver);
+    if (!std::strcmp(name, "cuCtxGetCurrent")) *fn = reinterpret_cast<void *>(fake_cuCtxGetCurrent);
+    if (!std::strcmp(name, "cuPointerGetAttribute")) *fn = reinterpret_cast<void *>(fake_cuPointerGetAttribute);
+    *r = cudaDriverEntryPointSuccess;
     return cudaSuccess;
 }
 

@@ -16,7 +16,8 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["reuse", "capture", "bound", "give_back", "counts_as_free", "threads"])
+@pytest.mark.parametrize("scenario", ["reuse", "capture", "bound", "give_back", "counts_as_free", "context_in_place",
+                                      "context_elsewhere", "no_driver", "threads"])
 def test_device_memory(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -1,5 +1,7 @@
 """The library's kept device memory, through the public entry points: what other threads, batches, the caller and a
 new context see of it.  (test_device_memory.py tests the same code on a runtime of the host.)"""
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -97,3 +99,28 @@ def test_kept_memory_is_bounded_and_given_back_on_request():
     assert T.trim_memory() > 0
     assert free - torch.cuda.mem_get_info()[0] <= 64 << 20
     assert T.trim_memory() == 0
+
+
+def test_a_new_context_after_a_device_reset_starts_afresh():
+    """A program that frees its handles and resets the device builds and runs on; nothing that was kept of the old
+    context (blocks, streams, kernel attributes) is used in the new one."""
+    code = """
+import ctypes, sys
+import numpy as np
+sys.path[:0] = %r
+import oracle as O, pytrav as T
+rt = ctypes.CDLL("libcudart.so.12")
+V = 1 << 14
+s, d, w = O.rmat(14, 4, seed=2)
+for k in range(3):
+    g = T.Graph.from_edges(V, s, d, w)
+    assert np.array_equal(g.bfs([1])[0], O.bfs_levels(V, s, d, 1)), k
+    want = O.dijkstra(V, s, d, w, 1)
+    for delta in (0.0, 0.1):
+        assert np.array_equal(g.sssp([1], delta=delta)[0].view(np.uint32), want.view(np.uint32)), (k, delta)
+    g.free()
+    assert rt.cudaDeviceReset() == 0
+print("fine")
+""" % (sys.path,)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "fine", r.stdout + r.stderr
