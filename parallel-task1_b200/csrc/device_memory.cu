@@ -17,6 +17,10 @@
 // would do the same, but CUDA refuses one while any of its streams is captured,
 // and the capture, another thread's perhaps, is lost.
 //
+// Host memory can run out too: an allocation then fails as one of the device's
+// does, and freeing allocates nothing (the list nodes move), since it happens in
+// destructors.
+//
 // Blocks and streams belong to the context they were made in, and are gone when
 // it ends (cudaDeviceReset).  So they are kept by context, and each context's
 // keeps hold a mark: an allocation whose buffer id, which no other allocation of
@@ -27,6 +31,7 @@
 #include <atomic>
 #include <list>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <vector>
 
@@ -58,7 +63,8 @@ struct Context {
 
 // never destroyed: handles may be freed while the process exits
 std::mutex &g_mu = *new std::mutex;
-std::unordered_map<void *, Block> &g_live = *new std::unordered_map<void *, Block>;  // blocks handed out
+std::list<Block> &g_live = *new std::list<Block>;  // blocks handed out, and where to find them
+std::unordered_map<void *, std::list<Block>::iterator> &g_live_at = *new std::unordered_map<void *, std::list<Block>::iterator>;
 std::unordered_map<cudaStream_t, unsigned long long> &g_live_streams =
     *new std::unordered_map<cudaStream_t, unsigned long long>;  // streams handed out, and their contexts' epochs
 std::list<Context> &g_contexts = *new std::list<Context>;
@@ -136,8 +142,14 @@ Context *context_here()
         return nullptr;
     }
     n.epoch = ++g_epochs;
-    n.streams.reserve(kKeepStreams);
-    g_contexts.push_back(n);
+    try {
+        g_contexts.push_back(n);
+        g_contexts.back().streams.reserve(kKeepStreams);
+    } catch (const std::bad_alloc &) {
+        while (!g_contexts.empty() && g_contexts.back().epoch == n.epoch) g_contexts.pop_back();
+        cudaFree(n.mark);
+        return nullptr;
+    }
     return &g_contexts.back();
 }
 
@@ -155,15 +167,14 @@ bool lives(unsigned long long epoch)
 }
 
 // Take idle blocks of a context out of its list, oldest first, until those left hold at most `keep` bytes.
-std::vector<void *> take_over(Context *c, size_t keep)
+std::list<Block> take_over(Context *c, size_t keep)
 {
     size_t held = 0;
     for (const Block &b : c->kept) held += b.bytes;
-    std::vector<void *> out;
+    std::list<Block> out;
     while (!c->kept.empty() && held > keep) {
         held -= c->kept.front().bytes;
-        out.push_back(c->kept.front().p);
-        c->kept.pop_front();
+        out.splice(out.end(), c->kept, c->kept.begin());
     }
     return out;
 }
@@ -204,9 +215,13 @@ cudaError_t dev_malloc_bytes(void **p, size_t bytes)
                     (best == c->kept.end() || it->bytes < best->bytes))
                     best = it;
             if (best != c->kept.end()) {
+                try {
+                    g_live_at.emplace(best->p, best);
+                } catch (const std::bad_alloc &) {
+                    return cudaErrorMemoryAllocation;
+                }
+                g_live.splice(g_live.end(), c->kept, best);
                 *p = best->p;
-                g_live[best->p] = *best;
-                c->kept.erase(best);
                 return cudaSuccess;
             }
         }
@@ -220,23 +235,32 @@ cudaError_t dev_malloc_bytes(void **p, size_t bytes)
         *p = nullptr;
         return e;
     }
+    std::list<Block> node;
     std::lock_guard<std::mutex> lock(g_mu);
-    g_live[*p] = Block{*p, bytes, current_device(), epoch};
+    try {
+        node.push_back(Block{*p, bytes, current_device(), epoch});
+        g_live_at[*p] = node.begin();
+    } catch (const std::bad_alloc &) {
+        cudaFree(*p);
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
+    g_live.splice(g_live.end(), node);
     return cudaSuccess;
 }
 
 size_t dev_trim()
 {
     size_t bytes = 0;
-    std::vector<void *> out;
+    std::list<Block> out;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        if (Context *c = context_here()) {
-            for (const Block &b : c->kept) bytes += b.bytes;
-            out = take_over(c, 0);
-        }
+        if (Context *c = context_here()) out = take_over(c, 0);
     }
-    for (void *q : out) cudaFree(q);
+    for (const Block &b : out) {
+        bytes += b.bytes;
+        cudaFree(b.p);
+    }
     return bytes;
 }
 
@@ -251,36 +275,37 @@ cudaError_t dev_free_bytes(size_t want, size_t *bytes)
 void dev_free(void *p, cudaStream_t st)
 {
     if (!p) return;
-    Block b{p, 0, -1, 0};
+    std::list<Block> node;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        auto it = g_live.find(p);
-        if (it != g_live.end()) {
-            b = it->second;
-            g_live.erase(it);
+        auto it = g_live_at.find(p);
+        if (it != g_live_at.end()) {
+            node.splice(node.end(), g_live, it->second);
+            g_live_at.erase(it);
         }
     }
-    if (b.device < 0) {
+    if (node.empty()) {
         cudaFree(p);
         return;
     }
+    const Block b = node.front();
     const int cur = current_device();
     if (cur != b.device) cudaSetDevice(b.device);
     // nothing may still read or write the block when it is handed on
     const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) cudaGetLastError();  // not the caller's next launch's
-    std::vector<void *> out;
+    std::list<Block> out;
     {
         std::lock_guard<std::mutex> lock(g_mu);
         Context *c = context_here();
         if (e == cudaSuccess && c && c->epoch == b.epoch && b.bytes <= kKeepBytes) {
             out = take_over(c, kKeepBytes - b.bytes);
-            c->kept.push_back(b);
+            c->kept.splice(c->kept.end(), node);
         } else if (lives(b.epoch)) {
-            out.push_back(p);
+            out.splice(out.end(), node);
         }
     }
-    for (void *q : out) cudaFree(q);
+    for (const Block &x : out) cudaFree(x.p);
     if (cur != b.device) cudaSetDevice(cur);
 }
 
@@ -295,7 +320,13 @@ cudaError_t stream_get(cudaStream_t *st)
         const cudaError_t e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
         if (e != cudaSuccess) return e;
     }
-    g_live_streams[*st] = c ? c->epoch : 0;
+    try {
+        g_live_streams[*st] = c ? c->epoch : 0;
+    } catch (const std::bad_alloc &) {
+        cudaStreamDestroy(*st);
+        *st = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
     return cudaSuccess;
 }
 

@@ -315,16 +315,18 @@ public:
     void add(T **p, int64_t n)
     {
         *p = nullptr;
-        parts_.push_back(Part{reinterpret_cast<void **>(p), bytes_});
+        if (n_ < kMost) parts_[n_] = Part{reinterpret_cast<void **>(p), bytes_};
+        n_++;
         bytes_ += (sizeof(T) * (size_t)(n > 0 ? n : 1) + 255) & ~(size_t)255;
     }
     cudaError_t commit()
     {
-        for (size_t i = 0; i + 1 < parts_.size(); i++)
+        if (n_ > kMost) return cudaErrorInvalidValue;
+        for (int i = 0; i + 1 < n_; i++)
             if (alloc_failure_due()) return cudaErrorMemoryAllocation;
         const cudaError_t e = dev_malloc_bytes(&mem_, bytes_);
         if (e != cudaSuccess) return e;
-        for (const Part &p : parts_) *p.at = static_cast<unsigned char *>(mem_) + p.offset;
+        for (int i = 0; i < n_; i++) *parts_[i].at = static_cast<unsigned char *>(mem_) + parts_[i].offset;
         return cudaSuccess;
     }
     void *release()
@@ -335,8 +337,10 @@ public:
     }
 
 private:
+    static constexpr int kMost = 24;  // arrays (on the stack: add() cannot fail)
     struct Part { void **at; size_t offset; };
-    std::vector<Part> parts_;
+    Part parts_[kMost];
+    int n_ = 0;
     size_t bytes_ = 0;
     void *mem_ = nullptr;
     cudaStream_t st_;

@@ -4,11 +4,26 @@
 #include "../parallel-task1_b200/csrc/device_memory.cu"
 
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <random>
 #include <thread>
 
 using namespace trav;
+
+// The library's host allocations that still succeed (-1: all).
+static std::atomic<int> g_host_left{-1};
+void *operator new(size_t n)
+{
+    if (!fake::inside && g_host_left >= 0 && g_host_left-- == 0) {
+        g_host_left = 0;
+        throw std::bad_alloc();
+    }
+    if (void *p = std::malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 static int g_bad = 0;
 #define CHECK(x)                                                      \
@@ -153,6 +168,39 @@ static void no_driver()
     CHECK(fake::count("stream destroy") == 1 && cudaGetLastError() == cudaSuccess);
 }
 
+// No host memory: allocations fail without a leak, and freeing needs none.
+static void host_memory()
+{
+    cudaStream_t a = stream(), b = nullptr;
+    void *p = get(10 * MB), *q = get(20 * MB), *r = nullptr;
+    dev_free(q, a);
+    for (int left = 0; left < 4; left++) {
+        const size_t used = fake::used;
+        g_host_left = left;
+        const cudaError_t e = dev_malloc_bytes(&r, 30 * MB);
+        g_host_left = -1;
+        CHECK(e == cudaSuccess ? r != nullptr : e == cudaErrorMemoryAllocation && !r && fake::used == used);
+        dev_free(r, a);
+        dev_trim();
+    }
+    dev_free(get(20 * MB), a);
+    g_host_left = 0;
+    CHECK(dev_malloc_bytes(&r, 20 * MB) == cudaErrorMemoryAllocation && !r);  // a kept block stays where it is
+    CHECK(stream_get(&b) == cudaErrorMemoryAllocation && !b);
+    dev_free(p, a);
+    stream_put(a);
+    g_host_left = -1;
+    CHECK(get(10 * MB) == p);
+    CHECK(stream() == a);
+    DevSlab s(a);
+    int *x[25];
+    for (int **i = x; i < x + 24; i++) s.add(i, 100);
+    CHECK(s.commit() == cudaSuccess && x[23] == x[0] + 23 * 128);
+    DevSlab t(a);
+    for (int *&i : x) t.add(&i, 100);
+    CHECK(t.commit() == cudaErrorInvalidValue && !x[24]);
+}
+
 // Several threads: no block has two owners.
 static void threads()
 {
@@ -204,7 +252,8 @@ int main(int argc, char **argv)
         void (*run)();
     } all[] = {{"reuse", reuse}, {"capture", capture}, {"bound", bound}, {"give_back", give_back},
                 {"counts_as_free", counts_as_free}, {"context_in_place", context_in_place},
-                {"context_elsewhere", context_elsewhere}, {"no_driver", no_driver}, {"threads", threads}};
+                {"context_elsewhere", context_elsewhere}, {"no_driver", no_driver}, {"host_memory", host_memory},
+                {"threads", threads}};
     for (const auto &s : all)
         if (argc == 2 && !std::strcmp(argv[1], s.name)) {
             s.run();

@@ -29,6 +29,12 @@ struct Stream {
 };
 
 inline std::mutex mu;
+inline thread_local int inside = 0;  // calls of this runtime on the thread's stack
+struct Entry {
+    std::lock_guard<std::mutex> lock{mu};
+    Entry() { inside++; }
+    ~Entry() { inside--; }
+};
 inline std::map<void *, Alloc> allocs;
 inline std::map<cudaStream_t, Stream> streams;  // key 0: the legacy stream
 inline std::vector<std::string> log;
@@ -67,7 +73,7 @@ extern "C" {
 
 cudaError_t cudaMalloc(void **p, size_t bytes)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     using namespace fake;
     log.push_back("malloc");
     current = true;
@@ -80,7 +86,7 @@ cudaError_t cudaMalloc(void **p, size_t bytes)
 }
 cudaError_t cudaFree(void *p)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     using namespace fake;
     current = true;
     if (!p) return cudaSuccess;
@@ -93,7 +99,7 @@ cudaError_t cudaFree(void *p)
 }
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     *f = fake::capacity - fake::used;
     *t = fake::capacity;
     return cudaSuccess;
@@ -102,14 +108,14 @@ cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError()
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     const cudaError_t e = fake::last;
     fake::last = cudaSuccess;
     return e;
 }
 cudaError_t cudaDeviceSynchronize()
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     using namespace fake;
     log.push_back("device wait");
     for (auto &s : streams)
@@ -119,7 +125,7 @@ cudaError_t cudaDeviceSynchronize()
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *st, unsigned)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     using namespace fake;
     static unsigned long long at = 0x1000;
     log.push_back("stream create");
@@ -129,7 +135,7 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *st, unsigned)
 }
 cudaError_t cudaStreamDestroy(cudaStream_t st)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     using namespace fake;
     log.push_back("stream destroy");
     if (!streams.erase(st)) log.push_back("destroyed a stream that is gone");
@@ -137,7 +143,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t st)
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t st)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     using namespace fake;
     if (st && !streams.count(st)) {
         log.push_back("waited for a stream that is gone");
@@ -155,7 +161,7 @@ CUresult fake_cuCtxGetCurrent(CUcontext *c)
 }
 CUresult fake_cuPointerGetAttribute(void *out, CUpointer_attribute what, CUdeviceptr p)
 {
-    std::lock_guard<std::mutex> lock(fake::mu);
+    fake::Entry entry;
     auto it = fake::allocs.find(reinterpret_cast<void *>(p));
     if (what != CU_POINTER_ATTRIBUTE_BUFFER_ID || it == fake::allocs.end()) return CUDA_ERROR_INVALID_VALUE;
     *static_cast<unsigned long long *>(out) = it->second.id;

@@ -17,7 +17,7 @@ def check(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["reuse", "capture", "bound", "give_back", "counts_as_free", "context_in_place",
-                                      "context_elsewhere", "no_driver", "threads"])
+                                      "context_elsewhere", "no_driver", "host_memory", "threads"])
 def test_device_memory(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
