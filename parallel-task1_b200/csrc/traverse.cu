@@ -2346,9 +2346,14 @@ int persistent_grid_size(int kind)
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const void *fn = kind == 0 ? (const void *)bfs_persistent<false>
-                   : kind == 1 ? (const void *)sssp_persistent<false> : (const void *)batch_persistent;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kBlock, 0);
+    // every kernel that is launched with this grid has to fit: the resuming ones need other registers
+    const void *const fns[3][2] = {{(const void *)bfs_persistent<false>, (const void *)bfs_persistent<true>},
+                                   {(const void *)sssp_persistent<false>, (const void *)sssp_persistent<true>},
+                                   {(const void *)batch_persistent, (const void *)batch_persistent}};
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fns[kind][0], kBlock, 0);
+    int other = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&other, fns[kind][1], kBlock, 0);
+    per = std::min(per, other);
     if (e != cudaSuccess || per < 1 || sms < 1) {
         cuda_fail(e == cudaSuccess ? cudaErrorInvalidConfiguration : e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
         return -1;
