@@ -1,6 +1,7 @@
 // C ABI of the traversal library (declared in include/trav.h).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -732,8 +733,9 @@ int trav_mlp_set_margin(trav_graph *g, int32_t kind, float margin)
 
 static __global__ void init_distances_kernel(float *d, int32_t V, int32_t s)
 {
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
-        d[i] = i == s ? 0.0f : FLT_MAX;
+    // (V may be near 2^31)
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)V; i += gridDim.x * blockDim.x)
+        d[i] = (int32_t)i == s ? 0.0f : FLT_MAX;
 }
 
 static __global__ void gather_bits_kernel(unsigned *value, const float *d, const int32_t *old_of_new, int32_t V)
@@ -747,7 +749,7 @@ int trav_init_distances_f32(float *d, int32_t vertices, int32_t source)
     TRY(check_device());
     if (!d || vertices < 1 || !is_device_ptr(d)) return bad("d must be a device array of vertices >= 1 floats");
     if (source < 0 || source >= vertices) return bad("source vertex out of range [0, V)");
-    init_distances_kernel<<<(vertices + 255) / 256 < 4096 ? (vertices + 255) / 256 : 4096, 256>>>(d, vertices, source);
+    init_distances_kernel<<<(int)std::min<int64_t>(((int64_t)vertices + 255) / 256, 4096), 256>>>(d, vertices, source);
     TRY_CUDA(cudaGetLastError());
     TRY_CUDA(cudaDeviceSynchronize());
     return TRAV_OK;

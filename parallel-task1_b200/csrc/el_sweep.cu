@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) el_reach_kernel(SweepArgs a)
         done = !changed_in(a, k);
     }
     if (!done) return;  // converged stays 0: the caller takes the CSR path
-    for (int v = gtid; v < a.V; v += nth) a.visited[v] = (__ldcg(&gr[v >> 5]) >> (v & 31)) & 1u;
+    for (unsigned v = (unsigned)gtid; v < (unsigned)a.V; v += (unsigned)nth)  // (V may be near 2^31)
+        a.visited[v] = (__ldcg(&gr[v >> 5]) >> (v & 31u)) & 1u;
     if (gtid == 0) a.ctl->converged = 1;
 }
 

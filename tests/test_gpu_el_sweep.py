@@ -101,3 +101,29 @@ def test_bad_edges_are_refused_and_nothing_is_written():
             T.bellman_ford_wrapper(*(torch.from_numpy(x).cuda() for x in (s, d2, w)), V, 99, 0, dist)
         assert e.value.code == T.TRAV_ERR_BAD_ARG and msg in str(e.value)
         assert bool((dist == 5.0).all())
+
+
+def test_the_largest_vertex_count():
+    """V = 2^31 - 1: vertex loops count past 2^31."""
+    import torch
+
+    V = (1 << 31) - 1
+    path = [0, V - 1, V - 2, 5, 1 << 30]
+    s, d = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (path[:-1], path[1:]))
+    w = torch.full((4,), 0.5, device="cuda")
+    vis = torch.full((V + 1,), 9, dtype=torch.uint8, device="cuda")
+    T.bfs_wrapper(s, d, V, 4, vis, 0)
+    assert vis[V].item() == 9 and vis[path].tolist() == [1] * 5 and int(vis[:V].sum(dtype=torch.int64)) == 5
+    trees = torch.zeros(V, dtype=torch.int32, device="cuda")
+    trees[5] = 1  # outside the pivot's tree, and on the way to the last vertex
+    pivot = torch.zeros(1, dtype=torch.int32, device="cuda")
+    T._check(T.lib().trav_reach_el_masked(s.data_ptr(), d.data_ptr(), V, 4, pivot.data_ptr(), trees.data_ptr(),
+                                          vis.data_ptr()))
+    assert vis[V].item() == 9 and vis[path].tolist() == [1, 1, 1, 0, 0] and int(vis[:V].sum(dtype=torch.int64)) == 3
+    del vis, trees
+    dist = torch.full((V + 1,), -7.0, device="cuda")
+    T.init_distances(dist, V, 0)
+    assert dist[V].item() == -7.0 and dist[0].item() == 0.0 and bool((dist[1:V] == float(FLT_MAX)).all())
+    T.bellman_ford_wrapper(s, d, w, V, 4, 0, dist)
+    assert dist[V].item() == -7.0 and dist[path].tolist() == [0.0, 0.5, 1.0, 1.5, 2.0]
+    assert int((dist[:V] < float(FLT_MAX)).sum()) == 5
