@@ -51,3 +51,22 @@ def test_distances_around_the_limits(V, E):
         assert np.array_equal(outs[k].cpu().numpy().view(np.uint32), want[k % 2])
     b.close()
     g.free()
+
+
+@pytest.mark.parametrize("V,E", [(1 << 13, 1 << 18), ((1 << 19) + 3, 9_000_000)])
+def test_pull_rounds_gather_sources_through_l1(V, E):
+    """All rows near, and only the first 8,192: the source's distance of a pulled edge may be old, and the result must
+    not be."""
+    s, d, w = _skewed(V, E, V + 1)
+    g = T.Graph.from_edges(V, s, d, w)
+    csr = O.csr(V, s, d, w)
+    deg = np.bincount(s, minlength=V)
+    order = np.argsort(-deg, kind="stable")
+    pulled = 0
+    for x in (int(order[0]), int(order[5]), int(np.flatnonzero(deg)[-1])):
+        ref = O.dijkstra(V, s, d, w, x, csr_arrays=csr).view(np.uint32)
+        for delta in (0.02, 0.1):
+            assert np.array_equal(g.sssp([x], delta=delta)[0].view(np.uint32), ref), (x, delta)
+            pulled += int(np.sum(g.last_phase_log()[0] == 7))
+    assert pulled > 0
+    g.free()
