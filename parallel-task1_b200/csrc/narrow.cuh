@@ -524,12 +524,37 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
             }
         } else if (cmd == kNarrowPull) {
             // bottom-up (graphs that run here alone): every unvisited vertex
-            // looks for a parent of the current level
+            // looks for a parent of the current level, a long in-row with its
+            // whole warp (500 dense vertices beside one with 4,500 in-edges from
+            // vertices that are never reached, whole call: 690 us four parents at
+            // a time by one thread, 83 us so, 172 us in the wide kernel)
             const int level = s.level_next - 1;
-            for (unsigned v = gtid; v < (unsigned)a.V; v += nth) {
-                if (__ldcg(&a.visited[v >> 5]) >> (v & 31u) & 1u) continue;
-                const int b = __ldg(&a.in_off[v]), end = __ldg(&a.in_off[v + 1]);
+            const unsigned lane = tid & 31u;
+            for (unsigned v = gtid; __any_sync(kFull, v < (unsigned)a.V); v += nth) {
+                const bool open = v < (unsigned)a.V && !(__ldcg(&a.visited[v >> 5]) >> (v & 31u) & 1u);
+                int b = open ? __ldg(&a.in_off[v]) : 0;
+                const int end = open ? __ldg(&a.in_off[v + 1]) : 0;
                 bool hit = false;
+                for (unsigned coop = __ballot_sync(kFull, end - b > kBuCoop); coop; coop &= coop - 1) {
+                    const int owner = __ffs(coop) - 1;
+                    const int rb = __shfl_sync(kFull, b, owner), re = __shfl_sync(kFull, end, owner);
+                    bool h = false;
+                    for (int e = rb; e < re && !__any_sync(kFull, h); e += 128) {
+                        int u[4];
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            const int k = e + 32 * j + (int)lane;
+                            u[j] = k < re ? __ldg(&a.in_adj[k]) : -1;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; j++) h |= u[j] >= 0 && (int)__ldcg(&a.value[u[j]]) == level;
+                    }
+                    h = __any_sync(kFull, h);
+                    if ((int)lane == owner) {
+                        hit = h;
+                        b = end;
+                    }
+                }
                 for (int e = b; e < end && !hit; e += 4) {
                     int u[4];
 #pragma unroll

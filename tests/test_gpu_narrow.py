@@ -117,3 +117,21 @@ def test_frontiers_of_one_width(width):
     s, d = np.concatenate(s).astype(np.int64), np.concatenate(d)
     rng = np.random.default_rng(width)
     _check(1 + n * width, s, d, (rng.integers(1, 20, len(s)) / 4).astype(np.float32), 0, deltas=(0.0, 1.0, 3.0))
+
+
+@pytest.mark.parametrize("where", ["apart", "first", "last"])
+@pytest.mark.parametrize("deg", [511, 512, 513, 640, 641, 4000])
+def test_long_in_rows_in_bottom_up_steps(deg, where):
+    """An in-row around the length from which a whole warp scans it: without a parent that is ever reached, with one
+    at its start, or at its end; beside rows of every lane's own."""
+    rng = np.random.default_rng(deg)
+    n = 400  # a dense part that is searched bottom-up, a hub, and `deg` sources of it
+    hub = n
+    s = np.concatenate([rng.integers(0, n, 20 * n), hub + 1 + np.arange(deg)])
+    d = np.concatenate([rng.integers(0, n, 20 * n), np.full(deg, hub)])
+    # in-rows are in the order of falling out-degree, then of ids
+    if where == "first":
+        s, d = np.concatenate([s, np.full(301, n - 1)]), np.concatenate([d, [hub], rng.integers(0, n, 300)])
+    elif where == "last":
+        s, d = np.concatenate([s, [3]]), np.concatenate([d, [hub + deg]])
+    _check(n + 1 + deg, s, d, rng.random(len(s), dtype=np.float32), 0, deltas=(0.0,))
