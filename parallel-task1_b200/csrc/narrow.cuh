@@ -524,20 +524,30 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
             }
         } else if (cmd == kNarrowPull) {
             // bottom-up (graphs that run here alone): every unvisited vertex
-            // looks for a parent of the current level, a long in-row with its
-            // whole warp (500 dense vertices beside one with 4,500 in-edges from
-            // vertices that are never reached, whole call: 690 us four parents at
-            // a time by one thread, 83 us so, 172 us in the wide kernel)
+            // looks for a parent of the current level, and a long in-row that has
+            // none among its first is left to the whole warp (500 dense vertices
+            // beside one with 4,500 in-edges from vertices that are never reached,
+            // whole call: 690 us four parents at a time by one thread, 82 us so, 172
+            // us in the wide kernel; 512 vertices of 512 edges, where nearly every
+            // first parent is one: four queries 131 us, and 145 with the warp at once)
+            constexpr int kOwn = 32;  // parents a lane looks at in a long row
             const int level = s.level_next - 1;
             const unsigned lane = tid & 31u;
             for (unsigned v = gtid; __any_sync(kFull, v < (unsigned)a.V); v += nth) {
                 const bool open = v < (unsigned)a.V && !(__ldcg(&a.visited[v >> 5]) >> (v & 31u) & 1u);
-                int b = open ? __ldg(&a.in_off[v]) : 0;
-                const int end = open ? __ldg(&a.in_off[v + 1]) : 0;
+                const int b = open ? __ldg(&a.in_off[v]) : 0, end = open ? __ldg(&a.in_off[v + 1]) : 0;
+                const int own = end - b > kBuCoop ? b + kOwn : end;
                 bool hit = false;
-                for (unsigned coop = __ballot_sync(kFull, end - b > kBuCoop); coop; coop &= coop - 1) {
+                for (int e = b; e < own && !hit; e += 4) {
+                    int u[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) u[j] = e + j < own ? __ldg(&a.in_adj[e + j]) : -1;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) hit |= u[j] >= 0 && (int)__ldcg(&a.value[u[j]]) == level;
+                }
+                for (unsigned coop = __ballot_sync(kFull, own < end && !hit); coop; coop &= coop - 1) {
                     const int owner = __ffs(coop) - 1;
-                    const int rb = __shfl_sync(kFull, b, owner), re = __shfl_sync(kFull, end, owner);
+                    const int rb = __shfl_sync(kFull, own, owner), re = __shfl_sync(kFull, end, owner);
                     bool h = false;
                     for (int e = rb; e < re && !__any_sync(kFull, h); e += 128) {
                         int u[4];
@@ -550,17 +560,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
                         for (int j = 0; j < 4; j++) h |= u[j] >= 0 && (int)__ldcg(&a.value[u[j]]) == level;
                     }
                     h = __any_sync(kFull, h);
-                    if ((int)lane == owner) {
-                        hit = h;
-                        b = end;
-                    }
-                }
-                for (int e = b; e < end && !hit; e += 4) {
-                    int u[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) u[j] = e + j < end ? __ldg(&a.in_adj[e + j]) : -1;
-#pragma unroll
-                    for (int j = 0; j < 4; j++) hit |= u[j] >= 0 && (int)__ldcg(&a.value[u[j]]) == level;
+                    if ((int)lane == owner) hit = h;
                 }
                 if (!hit) continue;
                 reinterpret_cast<int *>(a.value)[v] = level + 1;
