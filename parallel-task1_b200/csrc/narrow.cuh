@@ -28,14 +28,14 @@
 //
 // Rows of the frontier stay with the CTA that found them, or are dealt round
 // when they are unevenly spread; 2^g lanes to a row and
-// four edges to a lane at a time, with g from the mean row length: the edges,
-// gathers and atomics of a lane are in flight together.
+// four edges to a lane at a time, with g from the mean and the longest row: the
+// edges, gathers and atomics of a lane are in flight together.
 #pragma once
 
 // One CTA an SM.  512 threads: with 768 or 1024 SSSP on that grid takes 22.3 or
 // 24.3 ms instead of 18.3 (the warps without a row still step through the
 // phase's bookkeeping).
-constexpr int kNarrowThreads = 512;
+constexpr int kNarrowBits = 9, kNarrowThreads = 1 << kNarrowBits;
 constexpr int kNarrowCtas = 16;         // CTAs of the cluster (8 where the device cannot place 16)
 constexpr int kNarrowRows = 5120;       // rows a CTA's queue holds
 // Edges of the largest narrow phase.  The line is not sharp: with 16k, 64k or
@@ -219,11 +219,20 @@ __device__ __forceinline__ bool narrow_deal(unsigned most, unsigned units, unsig
     return most > units / C + units / (4 * C) + 16u;
 }
 
-// Lanes per row (as a power of two) for rows of edges / rows edges on average: four edges a lane.
-__device__ __forceinline__ int narrow_lanes(unsigned rows, unsigned edges)
+// Lanes per unit, as a power of two: four edges a lane for units of the mean
+// length, at most a warp; and more, up to a CTA's threads, while the longest unit,
+// which is the phase's chain, takes more rounds than there are over the `most`
+// units that 2^t threads share (a CTA's, or dealt round the cluster's).  On the
+// critical path of every phase: with a formula (count of leading zeros) in place
+// of the loops, which end at once on rows of four edges, the grid's SSSP took 3.5%
+// longer.  Whole calls, with and without the second loop: SSSP from the hub of a
+// star with 5,000 leaves, delta 0.1, 197 us and 617 (258 in the wide kernel); four
+// Bellman-Ford queries on RMAT, 2,048 vertices and 8,192 edges, 353 and 750 (455).
+__device__ __forceinline__ int narrow_lanes(unsigned units, unsigned edges, unsigned longest, unsigned most, int t)
 {
     int g = 0;
-    while (g < 5 && (edges >> (g + 2)) > rows) g++;
+    while (g < 5 && (edges >> (g + 2)) > units) g++;
+    while (g < kNarrowBits && ((int)longest - 1 >> (g + 2)) > (int)(most << g >> t)) g++;
     return g;
 }
 
@@ -372,6 +381,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
     NarrowShared &s = narrow();
     const unsigned C = cluster_size(), rank = cluster_rank(), tid = threadIdx.x;
     const unsigned gtid = tid * C + rank, nth = C * kNarrowThreads;  // consecutive units go to different CTAs
+    const int cluster_bits = kNarrowBits + 31 - __clz((int)C);
     Ctl *ctl = a.ctl;
     const int src = a.source;
     const bool own = a.V <= kNarrowOwn;
@@ -396,6 +406,8 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
     for (int p = 0;; p++) {
         if (tid < 32) {
             const NarrowTotal t = narrow_totals(p % 3);
+            const bool deal = narrow_deal(t.most, t.units, C);
+            const int lanes = narrow_lanes(t.units, t.edges, t.longest, deal ? t.units : t.most, deal ? cluster_bits : kNarrowBits);
             narrow_shares(t.rank.rows, t.rank.segs);
             const unsigned long long done_nf = nf;
             if (p > 0) {
@@ -420,8 +432,8 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) bfs_narrow(const __grid_con
             if (tid == 0) {
                 s.cmd = cmd;
                 s.rows = t.units;
-                s.g = narrow_lanes(t.units, t.edges);
-                s.dealt = narrow_deal(t.most, t.units, C);
+                s.dealt = deal;
+                s.g = lanes;
                 s.in = p & 1;
                 s.ring = (p + 1) % 3;
                 s.level_next = L + 1;
@@ -673,6 +685,7 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
     NarrowShared &s = narrow();
     const unsigned C = cluster_size(), rank = cluster_rank(), tid = threadIdx.x, lane = tid & 31u;
     const unsigned gtid = tid * C + rank, nth = C * kNarrowThreads;
+    const int cluster_bits = kNarrowBits + 31 - __clz((int)C);
     Ctl *ctl = a.ctl;
     const int src = a.source;
     const bool own = a.V <= kNarrowOwn;
@@ -744,7 +757,12 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                 cmd = kNarrowDone;
             }
             if (cmd != kNarrowDone && steps + buckets >= a.max_steps) cmd = kNarrowBudget;
-            narrow_shares(cmd == kNarrowHeavy ? nheavy : t.rank.rows, cmd == kNarrowHeavy ? 0u : t.rank.segs);
+            const bool hv = cmd == kNarrowHeavy;
+            const bool deal = narrow_deal(hv ? max_heavy : t.most, hv ? heavy : t.units, C);
+            const unsigned n_units = hv ? heavy : t.units;
+            const int lanes = narrow_lanes(n_units, hv ? heavy_edges : t.edges, hv ? heavy_longest : t.longest,
+                                           deal ? n_units : hv ? max_heavy : t.most, deal ? cluster_bits : kNarrowBits);
+            narrow_shares(hv ? nheavy : t.rank.rows, hv ? 0u : t.rank.segs);
             const unsigned mine = __shfl_sync(kFull, nheavy, (int)rank);
             if (cmd == kNarrowHeavy) nheavy = hedges = hlongest = 0;  // the list is used up; the other one starts empty
             int option = -1;
@@ -779,8 +797,8 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                 s.far_buf = p & 1;
                 s.far_pile = fcur;
                 s.hbase = cmd == kNarrowHeavy ? 0u : mine;
-                s.dealt = cmd == kNarrowHeavy ? narrow_deal(max_heavy, heavy, C) : narrow_deal(t.most, t.units, C);
-                s.g = cmd == kNarrowHeavy ? narrow_lanes(heavy, heavy_edges) : narrow_lanes(t.units, t.edges);
+                s.dealt = deal;
+                s.g = lanes;
                 s.in = p & 1;
                 s.ring = (p + 1) % 3;
                 s.thr = thr;

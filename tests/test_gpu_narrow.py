@@ -135,3 +135,14 @@ def test_long_in_rows_in_bottom_up_steps(deg, where):
     elif where == "last":
         s, d = np.concatenate([s, [3]]), np.concatenate([d, [hub + deg]])
     _check(n + 1 + deg, s, d, rng.random(len(s), dtype=np.float32), 0, deltas=(0.0,))
+
+
+@pytest.mark.parametrize("n", [3, 4, 5, 8, 9, 127, 129, 1023, 2047, 2048, 2049, 4097, 5000])
+def test_one_long_heavy_row_among_short_ones(n):
+    """A star whose leaves point back: the hub's heavy row, of about 2 n / 3 edges, is expanded beside as many rows of
+    one edge as there are leaves in the bucket, and gets up to a whole block's lanes."""
+    leaf = 1 + np.arange(n)
+    s = np.concatenate([np.zeros(n), leaf, leaf])
+    d = np.concatenate([leaf, np.zeros(n), 1 + (leaf % n)])
+    rng = np.random.default_rng(n)
+    _check(n + 1, s, d, (rng.integers(0, 9, len(s)) / 8).astype(np.float32), 0, deltas=(0.0, 0.3))
