@@ -209,6 +209,19 @@ __global__ void weight_sum_kernel(int64_t E, const float *__restrict__ w, double
     if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
 }
 
+// The largest of the falling degrees, and how many are above `limit`.
+__global__ void degree_marks_kernel(int32_t V, const int32_t *__restrict__ deg, int32_t limit, int32_t *__restrict__ marks)
+{
+    int32_t lo = 0, hi = V;
+    while (lo < hi) {
+        const int32_t mid = lo + (hi - lo) / 2;
+        if (deg[mid] > limit) lo = mid + 1;
+        else hi = mid;
+    }
+    marks[0] = deg[0];
+    marks[1] = lo;
+}
+
 template <class T>
 struct DBuf {
     T *p = nullptr;
@@ -317,7 +330,7 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
     keep.add(&g.out_w, E);
     keep.add(&g.in_w, E);
     TRY_CUDA(keep.commit());
-    int32_t *out_deg, *in_deg, *ids, *deg_sorted, *out_deg_new, *in_deg_new, *dv;
+    int32_t *out_deg, *in_deg, *ids, *deg_sorted, *out_deg_new, *in_deg_new, *dv, *marks;
     float *iwt;
     unsigned long long *okeys, *ikeys, *skeys;
     double *part;
@@ -334,6 +347,7 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
     tmp.add(&dv, E);
     tmp.add(&iwt, E);
     tmp.add(&part, kWSumBlocks);
+    tmp.add(&marks, 2);
     size_t tb = 0, tb2 = 0, tb3 = 0, tb4 = 0;
     TRY_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, (int32_t *)nullptr, (int32_t *)nullptr,
                                                        (int32_t *)nullptr, (int32_t *)nullptr, (int)V, 0, 32, st));
@@ -381,8 +395,12 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
         low_bits_kernel<<<grid_for(E), 256, 0, st>>>(E, mask, skeys, g.in_adj);
         TRY_CUDA(cudaGetLastError());
     }
-    int32_t maxdeg = 0;
-    if (V > 0) TRY_CUDA(cudaMemcpyAsync(&maxdeg, deg_sorted, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    int32_t deg_marks[2] = {0, 0};
+    if (V > 0) {
+        degree_marks_kernel<<<1, 1, 0, st>>>(V, deg_sorted, kNarrowRows, marks);
+        TRY_CUDA(cudaGetLastError());
+        TRY_CUDA(cudaMemcpyAsync(deg_marks, marks, sizeof(deg_marks), cudaMemcpyDeviceToHost, st));
+    }
     double wsum = 0.0;
     if (E > 0) {
         weight_sum_kernel<<<kWSumBlocks, 256, 0, st>>>(E, g.out_w, part);
@@ -396,7 +414,8 @@ int build_graph_device(int32_t V, int64_t E, const int32_t *d_src, const int32_t
 
     g.V = V;
     g.E = E;
-    g.max_out_degree = maxdeg;
+    g.max_out_degree = deg_marks[0];
+    g.long_rows = deg_marks[1];
     g.mean_w = E > 0 ? (float)(wsum / (double)E) : 0.0f;
     g.mem = keep.release();
     *out = g;

@@ -37,7 +37,6 @@
 // phase's bookkeeping).
 constexpr int kNarrowBits = 9, kNarrowThreads = 1 << kNarrowBits;
 constexpr int kNarrowCtas = 16;         // CTAs of the cluster (8 where the device cannot place 16)
-constexpr int kNarrowRows = 5120;       // rows a CTA's queue holds
 // Edges of the largest narrow phase.  The line is not sharp: with 16k, 64k or
 // 128k the grid, a uniform graph of 1M vertices and RMAT scale 16 measure the
 // same, since growing frontiers pass through this range in one step.
@@ -65,7 +64,7 @@ struct alignas(16) NarrowCount {
 static_assert(sizeof(NarrowCount) == 48, "read as three 16-byte words");
 
 struct NarrowShared {
-    // frontier rows of two phases, then the further segments
+    // frontier rows of two phases (kNarrowRows at most), then the further segments
     int v[2][kNarrowRows + kNarrowSegs], begin[2][kNarrowRows + kNarrowSegs], len[2][kNarrowRows + kNarrowSegs];
     int heavy[2][kNarrowRows];               // SSSP heavy lists
     int far[2][kNarrowRows];                 // vertices for the far pile, of two phases

@@ -12,6 +12,7 @@ namespace trav {
 
 constexpr int kBlock = 256;       // threads per CTA of the persistent kernels
 constexpr int kWarps = kBlock / 32;
+constexpr int kNarrowRows = 5120;  // rows a CTA's queue of the narrow kernel holds (narrow.cuh)
 constexpr int kChunk = 512;       // edges per chunk item (two-phase expansion of the allocation-free BFS)
 constexpr int kBigDegree = 512;   // rows longer than this are split into chunks there
 constexpr int kSmallDeg = 32;     // one-phase expansion (default): rows up to this length go to the warp-tile queue
@@ -106,6 +107,7 @@ struct DevGraph {
     int32_t V = 0;
     int64_t E = 0;
     int32_t max_out_degree = 0;
+    int32_t long_rows = 0;        // vertices with more than kNarrowRows out-edges: 0 .. long_rows - 1
     float mean_w = 0.0f;          // mean edge weight (a schedule feature)
     int32_t *out_off = nullptr;   // V+1
     int32_t *out_adj = nullptr;   // E

@@ -2217,10 +2217,39 @@ int launch_cooperative(const void *fn, int grid, void **params, cudaStream_t st)
     return TRAV_OK;
 }
 
-// Edges up to which a graph of at most kNarrowRows vertices is left to the
-// narrow kernel alone: above, a phase of most of the edges would take its 16 SMs
-// longer than the whole device with its barriers.
-constexpr int64_t kNarrowAloneEdges = 1 << 18;
+// Whether a query is left to the narrow kernel alone: its queues must hold any
+// phase, so at most kNarrowRows vertices, and no phase may have so many edges
+// that its 16 SMs take longer than the whole device with its barriers.
+//
+// SSSP: in a Bellman-Ford round that may be all edges.  Four queries from 512 /
+// 2,048 / 5,000 vertices, in us, alone and only begun here:
+//   32,768 edges, RMAT  332, 431, 531 and 398, 457, 543
+//   65,536              548, 450, 568 and 423, 475, 501; uniform 373, 519, 608 and 432, 680, 630
+//   131,072             704, 784, 658 and 449, 483, 528; uniform 482, 632, 720 and 490, 565, 683
+// so 32,768 edges, and twice as many where no row is long (a skewed graph's
+// segments crowd in the block that found them, and rows that find no place stay
+// whole).  With buckets narrower than the mean weight a round has a few of the
+// edges (delta 0.1, 262,144 edges: RMAT 680, 1004, 1245 and 769, 1050, 1227; uniform
+// 435, 544, 755 and 465, 569, 810), if long rows can be cut at all.
+// BFS: a top-down step has at most 1 / alpha of the edges before it is taken
+// bottom-up, or all where the caller forces the direction.  Top-down only, three
+// queries on RMAT: 5,000 vertices, 40,000 edges 177 alone and 225 in the wide
+// kernel; 160,000 edges 304 and 216; 2,000 vertices, 262,144 edges 428 and 194.
+// Bottom-up steps are the narrow kernel's up to the 262,144 edges tested (123 and
+// 190).
+constexpr int64_t kNarrowAloneEdges = 1 << 18, kNarrowAloneRound = 1 << 15, kNarrowAlonePush = 1 << 16;
+constexpr int kNarrowEvenRow = 512;
+
+bool narrow_alone(int kind, const TravArgs &a)
+{
+    if (a.V > kNarrowRows || a.E > kNarrowAloneEdges) return false;
+    if (kind == 1) {
+        if (a.nlight && a.delta < a.mean_w && a.max_deg <= kNarrowRows) return true;
+        return a.E <= kNarrowAloneRound * (a.max_deg <= kNarrowEvenRow ? 2 : 1);
+    }
+    const double push = a.force_dir == 0 ? (double)a.E : a.force_dir == 1 ? (double)a.max_deg : (double)a.E / a.alpha;
+    return push <= (double)kNarrowAlonePush;
+}
 
 // CTAs of the narrow kernel's cluster on the current device: 16 (a
 // non-portable size) where the device can place it, else 8, else 0 (none).
@@ -2303,9 +2332,8 @@ int enqueue_persistent(int kind, TravArgs &args, int ctas, bool narrow, cudaStre
     if (narrow) {
         const int cluster = narrow_ctas(kind);
         if (cluster > 0) {
-            // Small graphs run in the narrow kernel alone: no phase of theirs can
-            // outgrow its queues, and the wide launch would only add its 5-8 us.
-            alone = args.V <= kNarrowRows && args.E <= kNarrowAloneEdges;
+            // small graphs run in the narrow kernel alone: the wide launch would only add its 5-8 us
+            alone = narrow_alone(kind, args);
             TRY(launch_narrow(kind, args, cluster, alone, st));
             resume = true;
         }
@@ -2579,7 +2607,10 @@ int launch_bfs(const DevGraph &g, Workspace *ws, int q, int32_t source_new, cons
     a.mlp_margin = ws->mlp_margin[0];
     a.plan = ws->plan[0];
     a.plan_len = ws->plan_len[0];
-    return enqueue_persistent(0, a, ws->grid[0], narrow_query(*ws, 0) && !mlp, st, ev0, ev1);
+    // A source whose row the queues would not hold begins in the wide kernel, as the narrow one would only hand it over
+    // (RMAT scale 18 from its first vertex 116 us, 109 so); and so does a small graph with too many edges to stay narrow.
+    const bool begins = narrow_alone(0, a) || (g.V > kNarrowRows && source_new >= g.long_rows);
+    return enqueue_persistent(0, a, ws->grid[0], narrow_query(*ws, 0) && !mlp && begins, st, ev0, ev1);
 }
 
 int launch_sssp(const DevGraph &g, Workspace *ws, int q, int32_t source_new, float delta, const float *mlp,
@@ -2618,7 +2649,8 @@ int launch_sssp(const DevGraph &g, Workspace *ws, int q, int32_t source_new, flo
     // scale 16, edge factor 16, Bellman-Ford: 5% slower; uniform degree 16: 3%
     // faster; grid of degree 4: 1.4 times as fast).
     const bool sparse = g.E <= (int64_t)kNarrowDegree * g.V || g.V <= kNarrowRows;
-    return enqueue_persistent(1, a, ws->grid[1], narrow_query(*ws, 1) && source_new >= 0 && sparse, st, ev0, ev1);
+    const bool begins = narrow_alone(1, a) || (source_new >= g.long_rows && sparse);
+    return enqueue_persistent(1, a, ws->grid[1], narrow_query(*ws, 1) && source_new >= 0 && begins, st, ev0, ev1);
 }
 
 // Byte accounting of query q, which must be the last query run (its results

@@ -146,3 +146,18 @@ def test_one_long_heavy_row_among_short_ones(n):
     d = np.concatenate([leaf, np.zeros(n), 1 + (leaf % n)])
     rng = np.random.default_rng(n)
     _check(n + 1, s, d, (rng.integers(0, 9, len(s)) / 8).astype(np.float32), 0, deltas=(0.0, 0.3))
+
+
+@pytest.mark.parametrize("V,E,hub", [(5120, 32_768, 0), (5120, 32_769, 0), (5120, 65_536, 0), (5120, 65_537, 0),
+                                     (3000, 65_536, 512), (3000, 65_536, 513), (3000, 262_144, 5120),
+                                     (3000, 262_144, 5121), (3000, 262_145, 0), (20_000, 60_000, 5120),
+                                     (20_000, 60_000, 5121)])
+def test_queries_at_the_limits_of_where_they_run(V, E, hub):
+    """Edge counts and longest rows around those that decide whether a query runs in the narrow kernel alone, begins
+    there, or runs in the wide kernel; from the vertex of the longest row and from another, with forced directions."""
+    rng = np.random.default_rng(E + hub)
+    n = E - hub
+    s, d = np.concatenate([np.arange(n) % (V - 1) + 1, np.zeros(hub)]), rng.integers(0, V, E)
+    w = rng.random(E, dtype=np.float32)  # mean weight 0.5
+    for src in (0, 7):
+        _check(V, s, d, w, src, deltas=(0.0, 0.1, 0.6))
