@@ -161,3 +161,34 @@ def test_queries_at_the_limits_of_where_they_run(V, E, hub):
     w = rng.random(E, dtype=np.float32)  # mean weight 0.5
     for src in (0, 7):
         _check(V, s, d, w, src, deltas=(0.0, 0.1, 0.6))
+
+
+@pytest
+
+@pytest.mark.parametrize("hubs", [1, 8, 9, 10, 12])
+def test_far_vertices_of_one_block_are_written_out_in_time(hubs):
+    """A chain of hubs, each with a heavy row of 4,900 far leaves that two or three blocks expand, one bucket a hub.
+    From the tenth on, the pile in memory, shared out over 16 blocks, and the 2,048 vertices that a block has staged
+    could overflow its queue in the next bucket opening, and are written out first.  That is no phase of the query:
+    the log is the one of the wide kernel."""
+    leaves = 4900
+    V = hubs * (1 + leaves)
+    hub = np.arange(hubs)
+    s = np.concatenate([np.repeat(hub, leaves), hub[:-1]]).astype(np.int32)
+    d = np.concatenate([np.arange(hubs, V), hub[1:]]).astype(np.int32)
+    w = np.concatenate([np.full(hubs * leaves, 30.0), np.full(hubs - 1, 1.5)]).astype(np.float32)
+    want = []
+    for i in range(hubs):
+        want += [(5, 1), (4, (i + 1) * leaves + (i + 1 < hubs))]
+    want += [(4, i * leaves) for i in range(hubs - 1, 0, -1)]
+    g = T.Graph.from_edges(V, s, d, w)
+    ref = O.dijkstra(V, s, d, w, 0).view(np.uint32)
+    for ctas in (0, 5):  # 0: begins in the narrow kernel; the caller's shape: wide only
+        g.set_grid(1, ctas)
+        assert np.array_equal(g.sssp([0], delta=1.0)[0].view(np.uint32), ref)
+        kind, size, end_us, _ = g.last_phase_log()
+        # (the wide kernel may check for pulling, and pull, in a heavy round)
+        got = [(5 if k == 7 else int(k), int(x)) for k, x in zip(kind, size) if k != 6]
+        assert got == want, ctas
+        assert np.all(np.diff(end_us) >= 0)
+    g.free()
