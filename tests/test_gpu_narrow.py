@@ -163,8 +163,6 @@ def test_queries_at_the_limits_of_where_they_run(V, E, hub):
         _check(V, s, d, w, src, deltas=(0.0, 0.1, 0.6))
 
 
-@pytest
-
 @pytest.mark.parametrize("hubs", [1, 8, 9, 10, 12])
 def test_far_vertices_of_one_block_are_written_out_in_time(hubs):
     """A chain of hubs, each with a heavy row of 4,900 far leaves that two or three blocks expand, one bucket a hub.
