@@ -995,6 +995,8 @@ struct BfsPush {
     // gathers of a top-down step on a skewed graph; with every step top-down, RMAT
     // scale 16 takes 114 us instead of 172, scale 18 180 instead of 315, scale 21
     // 420 instead of 2675; four Beamer queries at scale 23 1605 instead of 1838.
+    // In a batch it is even: 512 queries on 64 small graphs 2.00 ms and 2.00, 16 at
+    // scale 21 1.50 and 1.52, 32 at scale 18 596 us and 605 (teams of 16: 484, 481).
     __device__ __forceinline__ unsigned visited_word(int v) const
     {
         unsigned w;
@@ -2645,9 +2647,15 @@ int launch_sssp(const DevGraph &g, Workspace *ws, int q, int32_t source_new, flo
     a.plan = ws->plan[1];
     a.plan_len = ws->plan_len[1];
     // On denser graphs the second or third round outgrows the narrow kernel, and
-    // handing over the hubs' heavy rows costs more than its rounds saved (RMAT
-    // scale 16, edge factor 16, Bellman-Ford: 5% slower; uniform degree 16: 3%
-    // faster; grid of degree 4: 1.4 times as fast).
+    // handing over costs more than its rounds saved, for Bellman-Ford on skewed
+    // graphs before all.  Begun in the narrow kernel against the wide one alone,
+    // four queries, RMAT / uniform of mean degree 4, 8 and 16:
+    //   2^17 vertices, Bellman-Ford   +3% / -1%, +4% / +2%, +10% / 0
+    //   2^17 vertices, delta 0.1      -6% / -17%, -4% / -14%, -3% / -13%
+    //   2^20 vertices, Bellman-Ford   +3% / 0, +2% / 0, +4% / 0
+    //   2^20 vertices, delta 0.1      -4% / -11%, -3% / -10%, -2% / -9%
+    // and a grid of mean degree 4, delta 80, -33%.  The line is where the gain of
+    // the one has come down to a few times the loss of the other.
     const bool sparse = g.E <= (int64_t)kNarrowDegree * g.V || g.V <= kNarrowRows;
     const bool begins = narrow_alone(1, a) || (source_new >= g.long_rows && sparse);
     return enqueue_persistent(1, a, ws->grid[1], narrow_query(*ws, 1) && source_new >= 0 && begins, st, ev0, ev1);
