@@ -944,8 +944,8 @@ __global__ void __launch_bounds__(kNarrowThreads, 1) sssp_narrow(const __grid_co
                                 const bool below = od < bound;
                                 push[j] = ((cls & kClsLight) && !(below && orr >= round_) ? 1u : 0u) |
                                           ((cls & kClsHeavy) && !(below && orr >= s.h_start) ? 2u : 0u);
-                            } else if (!(orr >= s.f_start)) {
-                                push[j] = 4u;
+                            } else {
+                                push[j] = orr >= s.f_start ? 0u : 4u;
                                 n.far_key = max(n.far_key, 0x7fffffff - __float_as_int(nd[j]));
                             }
                         }

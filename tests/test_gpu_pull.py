@@ -73,3 +73,44 @@ def test_pull_in_batch_matches_oracle(skewed):
     for src, out in zip(sources, outs):
         assert np.array_equal(_bits(out.cpu().numpy()), _bits(want[src])), src
     b.close()
+
+
+def test_pull_reaches_below_the_lowest_recorded_far_distance():
+    """Vertex 2 joins the far pile at 3.4 and is improved to 2.2 there, which the pile's lowest distance does not
+    follow; its heavy edge gives vertex 3 a distance (4.3) that lies below that record plus delta, and vertex 3 holds
+    5.0.  The heavy round pulls (nothing is left to pull over if vertex 3 is taken for settled)."""
+    import torch
+
+    s, d = np.array([0, 1, 0, 0, 2], np.int32), np.array([1, 2, 2, 3, 3], np.int32)
+    w = np.array([1.9, 1.5, 2.2, 5.0, 2.1], np.float32)
+    want = O.dijkstra(4, s, d, w, 0)
+    assert want[3] == np.float32(2.2) + np.float32(2.1)
+    g = T.Graph.from_edges(4, s, d, w)
+    out = torch.empty(4, dtype=torch.float32, device="cuda")
+    b = T.Batch([g])
+    b.run([(0, 1, 0, 2.0, T.SCHEDULE_PLAIN, out)])
+    for ctas in (0, 5):  # begins in the narrow kernel; the caller's shape: the wide kernel only
+        g.set_grid(1, ctas)
+        assert np.array_equal(_bits(g.sssp([0], delta=2.0)[0]), _bits(want)), ctas
+    assert np.array_equal(_bits(out.cpu().numpy()), _bits(want))
+    b.close()
+    g.free()
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_pull_in_the_wide_kernel_on_small_dense_graphs(seed):
+    """Whole weights (many ties and improvements in the far pile), wide and narrow buckets in turn."""
+    rng = np.random.default_rng(seed)
+    for _ in range(40):
+        V = int(rng.integers(4, 60))
+        E = int(rng.integers(V, 100 * V))
+        s, d = (rng.integers(0, V, E).astype(np.int32) for _ in range(2))
+        w = rng.integers(1, 100, E).astype(np.float32)
+        g = T.Graph.from_edges(V, s, d, w)
+        g.set_grid(1, 4)
+        src = int(s[0])
+        want = _bits(O.dijkstra(V, s, d, w, src))
+        for delta in (2.0, 9.0):
+            g.set_plan(1, rng.integers(0, 4, 64).astype(np.uint8))
+            assert np.array_equal(_bits(g.sssp([src], delta=delta)[0]), want), (V, E, delta)
+        g.free()
