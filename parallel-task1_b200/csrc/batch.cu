@@ -145,7 +145,9 @@ int ensure_teams(trav_batch *b, int teams)
         w.hch1 = c[3];
         w.ctl = b->ctl + t;
     }
-    TRY_CUDA(cudaMemcpy(b->d_teams, h.data(), sizeof(TeamWs) * (size_t)teams, cudaMemcpyHostToDevice));
+    // on the stream of the kernel that reads it (see trav_mlp_set)
+    TRY_CUDA(cudaMemcpyAsync(b->d_teams, h.data(), sizeof(TeamWs) * (size_t)teams, cudaMemcpyHostToDevice, b->st));
+    TRY_CUDA(cudaStreamSynchronize(b->st));
     b->teams_alloc = teams;
     return TRAV_OK;
 }

@@ -108,8 +108,8 @@ void destroy(trav_graph *h)
     for (cudaEvent_t e : h->ev) cudaEventDestroy(e);
     for (auto &c : h->cap)
         if (c.exec) cudaGraphExecDestroy(c.exec);
-    dev_free(h->mlp[0], nullptr);  // written on the legacy stream; its readers have been waited for
-    dev_free(h->mlp[1], nullptr);
+    dev_free(h->mlp[0], h->st);
+    dev_free(h->mlp[1], h->st);
     stream_put(h->cst);
     stream_put(h->own_st);
     delete h;
@@ -626,12 +626,13 @@ int trav_set_plan(trav_graph *g, int32_t kind, const uint8_t *plan, int32_t n)
     if (n < 0 || (n > 0 && !plan)) return bad("plan must hold n >= 0 entries");
     TRY_CUDA(cudaSetDevice(g->device));
     TRY_CUDA(cudaStreamSynchronize(g->st));
-    dev_free(g->ws.plan[kind], nullptr);  // written on the legacy stream
+    dev_free(g->ws.plan[kind], g->st);
     g->ws.plan[kind] = nullptr;
     g->ws.plan_len[kind] = 0;
     if (n == 0) return TRAV_OK;
     TRY_CUDA(dev_malloc(&g->ws.plan[kind], (size_t)n));
-    TRY_CUDA(cudaMemcpy(g->ws.plan[kind], plan, (size_t)n, cudaMemcpyHostToDevice));
+    TRY_CUDA(cudaMemcpyAsync(g->ws.plan[kind], plan, (size_t)n, cudaMemcpyHostToDevice, g->st));  // as in trav_mlp_set
+    TRY_CUDA(cudaStreamSynchronize(g->st));
     g->ws.plan_len[kind] = n;
     return TRAV_OK;
 }
@@ -714,7 +715,10 @@ int trav_mlp_set(trav_graph *g, int32_t kind, const float *params, int32_t count
         if (!std::isfinite(params[i])) return bad("MLP parameters must be finite");
     TRY_CUDA(cudaSetDevice(g->device));
     if (!g->mlp[kind]) TRY_CUDA(dev_malloc(&g->mlp[kind], sizeof(float) * (size_t)count));
-    TRY_CUDA(cudaMemcpy(g->mlp[kind], params, sizeof(float) * (size_t)count, cudaMemcpyHostToDevice));
+    // On the handle's stream: cudaMemcpy of pageable memory returns before its last
+    // bytes have arrived, and kernels of this stream do not wait for the legacy one.
+    TRY_CUDA(cudaMemcpyAsync(g->mlp[kind], params, sizeof(float) * (size_t)count, cudaMemcpyHostToDevice, g->st));
+    TRY_CUDA(cudaStreamSynchronize(g->st));
     return TRAV_OK;
 }
 

@@ -2538,8 +2538,8 @@ void workspace_free(Workspace *ws, cudaStream_t st)
     dev_free(ws->mem, st);
     light_rows_free(&ws->light, st);
     dev_free(ws->ctl, st);
-    dev_free(ws->plan[0], nullptr);  // written on the legacy stream
-    dev_free(ws->plan[1], nullptr);
+    dev_free(ws->plan[0], st);
+    dev_free(ws->plan[1], st);
     *ws = Workspace{};
 }
 

@@ -119,3 +119,26 @@ def test_cuda_graph_capture_replays_same_results(graph):
         assert np.array_equal(g.sssp(srcs, delta=0.05).view(np.uint32), ref_d.view(np.uint32))
     finally:
         g.set_capture(False)
+
+
+def test_a_query_takes_the_network_that_was_set_just_before():
+    """The decisions of a query are those of the network set in the call before it, by its features and the network's
+    formula on the host, whatever network was there before."""
+    from pytrav import learn
+
+    s, d, w = O.rmat(13, 8, seed=6)
+    g = T.Graph.from_edges(1 << 13, s, d, w)
+    src = int(np.bincount(s, minlength=1 << 13).argmax())
+    nets = [np.random.default_rng(k).normal(scale=2.0, size=T.mlp_param_count(1)).astype(np.float32) for k in range(4)]
+    checked = 0
+    for k in range(400):
+        p = nets[(k * 7 + k // 5) % 4]
+        g.set_mlp(1, p)
+        g.sssp([src], delta=0.02, schedule=T.SCHEDULE_LEARNED)
+        x, choice = g.last_decisions()[:2]
+        z = np.sort(learn.logits(1, p, x), axis=1)
+        clear = z[:, -1] - z[:, -2] > 1e-2
+        assert np.array_equal(np.argmax(learn.logits(1, p, x), axis=1)[clear], choice[clear]), k
+        checked += int(clear.sum())
+    assert checked > 400
+    g.free()
