@@ -1297,7 +1297,6 @@ struct SsspVisit {
         }
         p.ndef = base;
         bool light = false, heavy = false, far = false;
-        int far_key = 0;
         if (ok) {
             const unsigned long long old = atomicMin(&a->dist[v], pack_dist(nd, round << kClsBits | cls));
             const float od = dist_of(old);
@@ -1309,17 +1308,13 @@ struct SsspVisit {
                     heavy = (cls & kClsHeavy) && !(seen_below && orr >= h_start);
                 } else {
                     far = !(orr >= f_start);  // od > nd >= thr
-                    // the pile's lowest distance, also where this vertex is in the pile already: pull rounds
-                    // take it for a lower bound of the bucket's distances
-                    far_key = 0x7fffffff - __float_as_int(nd);
                 }
             }
         }
         const unsigned big_len = (unsigned)a->small_deg + 1u;  // any length that classifies as a long row
         push(p, 0, light, v, cls & kClsLightBig ? big_len : 1u);
         push(p, 1, heavy, v, cls & kClsHeavyBig ? big_len : 1u);
-        p.far_key = max(p.far_key, far_key);
-        push_far(p, far, v, far_key);
+        push_far(p, far, v, far ? 0x7fffffff - __float_as_int(nd) : 0);
         if (kHoldSlack >= 0.0f && light) p.light_key = max(p.light_key, 0x7fffffff - __float_as_int(nd));
     }
 };
@@ -1342,6 +1337,10 @@ __device__ __forceinline__ void init_counters(CtaCounters &cc)
 // Shared memory of one query's CTA (the bodies below run inside the
 // single-query kernels and inside the batch kernel).
 struct QueryShared {
+    // SSSP: lower bound of the current bucket, written by thread 0, read after the next barrier.  (Bellman-Ford from
+    // four sources on RMAT, 7.2 M vertices and 173 M edges, takes 25.4 ms with it here, and 27.5 with it in a register
+    // or at the end, where the arrays after it fall on other banks; 26.6 before pull rounds needed it.)
+    float lo;
     float mlp[kMlpMaxParams];  // the schedule network, copied in when the query has one
     WarpStage wst[kWarps];
     CtaCounters cc;
@@ -1693,7 +1692,7 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
     unsigned long long far_len = 0;
     int min_far = (int)kFltMaxBits;
     float thr = a.delta > 0.0f ? a.delta : INFINITY;
-    float lo = 0.0f;                        // lower bound of the current bucket
+    if (threadIdx.x == 0) sh.lo = 0.0f;     // lower bound of the current bucket
     int cur = 0, hcur = 0, fcur = 0;
 
     unsigned h_start = 1, f_start = 1;      // rounds the heavy list / far pile began in
@@ -1714,7 +1713,7 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
         far_len = r.far_len;
         min_far = r.min_far;
         thr = r.thr;
-        lo = r.lo;
+        if (threadIdx.x == 0) sh.lo = r.lo;
         fcur = r.fcur;
         h_start = r.h_start;
         f_start = r.f_start;
@@ -1831,16 +1830,17 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
             // phase first lists the vertices that a heavy edge could still improve, in the idle frontier buffer,
             // and counts their in-edges.  If they are fewer than half the heavy edges, the round pulls: it scans
             // those in-rows, and every in-edge u -> v relaxes v from u's distance, instead of pushing the heavy
-            // list's out-rows.  The heavy list lies at or above the bucket's lower bound lo, the lowest distance in the
-            // far pile that it opened with (the bound of the bucket before lists more vertices: RMAT scale 23 2.77 ms
-            // instead of 2.30, 512 queries on 64 graphs 6.38 instead of 5.26), and a heavy edge
+            // list's out-rows.  The heavy list lies at or above the bucket's lower bound lo, the lowest distance that it
+            // opened with (not min_far, which does not follow improvements of what is in the far pile already; and the
+            // bound of the bucket before lists more vertices: RMAT scale 23 2.77 ms instead of 2.30, 512 queries on 64
+            // graphs 6.38 instead of 5.26), and a heavy edge
             // weighs at least delta, so a heavy candidate is at least fl(lo + delta): a vertex at or below that
             // cannot improve, and every other vertex is in the list.
             bool pull = false;
             unsigned pq = 0, pch = 0;
             const double heavy_est = (double)hch * a.item + (double)hq * (0.5 * a.small_deg + 1.0);
             if (a.in_w && heavy_est * kPullCheck > (double)a.E) {
-                const float reach = __fadd_rn(lo, a.delta);
+                const float reach = __fadd_rn(sh.lo, a.delta);
                 clear_ahead(a, ph);
                 const FrontierOut lout{{(cur ? a.q0 : a.q1), nullptr}, {(cur ? a.chunks0 : a.chunks1), nullptr},
                                        {0u, 0u}, {0u, 0u}, {kPartIn, kPartIn}, nullptr, 0u, &ctl->slot[ph % kSlots]};
@@ -1915,7 +1915,6 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
             __syncthreads();
             const float told = thr;
             thr = s_delta;  // the new bound, computed once above (same inputs in every CTA)
-            lo = fmaxf(told, __int_as_float(min_far));
             const int32_t *fp = fcur ? a.far1 : a.far0;
             clear_ahead(a, ph);
             // the (empty) frontier and heavy list receive the entries of the new bucket
@@ -1930,6 +1929,7 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
             Pusher p = make_pusher(a, out, mys);
             const unsigned round = (unsigned)ph;
             h_start = f_start = round;  // the heavy list and the far pile begin again here
+            int lo_key = 0;             // max of 0x7fffffff - bits(d) over what opens the bucket
             for (unsigned long long base = (unsigned long long)gwarp * 32; base < far_len;
                  base += (unsigned long long)nwarps * 32) {
                 const unsigned long long i = base + lane_id();
@@ -1943,17 +1943,22 @@ __device__ __forceinline__ int sssp_query(const TravArgs &a, QueryShared &sh, De
                 const bool light = in_bucket && (cls & kClsLight);
                 const bool heavy = in_bucket && (cls & kClsHeavy);
                 const bool keep = valid && d >= thr;
+                if (in_bucket) lo_key = max(lo_key, 0x7fffffff - __float_as_int(d));
                 if (in_bucket || keep) atomicMax(&a.dist[v], pack_dist(d, round << kClsBits | cls));
                 push(p, 0, light, v, cls & kClsLightBig ? big_len : 1u);
                 push(p, 1, heavy, v, cls & kClsHeavyBig ? big_len : 1u);
                 push_far(p, keep, v, keep ? 0x7fffffff - __float_as_int(d) : 0);
             }
+            // the slot's mf carries it, as it carries the lowest distance of a light frontier
+            lo_key = __reduce_max_sync(kFull, lo_key);
+            if (lane_id() == 0 && lo_key) atomicMax(&cc.light_key, lo_key);
             finish_phase(p, cc);
             if (!grid_sync(a, ph, &s_view)) return -1;
             lg.scanned += s_view.scanned;
             log_phase(ctl, lg, 4, (unsigned)far_len);
             const SlotView s0 = s_view;
             hold_above = INFINITY;  // a bucket's first round expands everything it opened with
+            if (threadIdx.x == 0 && s0.mf) sh.lo = __int_as_float(0x7fffffff - (int)s0.mf);  // (else the bucket is empty)
             ph++;
             nq = s0.q_add;
             nch = s0.chunk_add;
